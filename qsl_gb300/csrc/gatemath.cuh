@@ -11,6 +11,7 @@
 
 #include "qslc_internal.cuh"
 #include "dpemu.cuh"
+#include "lean.cuh"
 
 #include <cmath>
 #include <cstdlib>
@@ -24,6 +25,8 @@ struct Coef {
     emu::MulConst kc, ks;   // c and s decoded for the full integer path (double only)
     emu::MulK mc, ms;       // c and s decoded for the integer products of the mixed path
     emu::DivConst kd;       // c as a divisor (Hadamard)
+    emu::LeanK lc, ls;      // c and s for easy operands (lean.cuh)
+    emu::LeanDiv ld;        // c as a divisor of easy operands
 };
 
 // How one gate output RN(RN(a*k1) +- RN(b*k2)) is computed (complex128):
@@ -135,7 +138,7 @@ __device__ __forceinline__ T dot2m(unsigned mode, T a, T k1, const emu::MulConst
 }
 
 enum PairOp { P_SWAP, P_Y, P_H, P_RX, P_RY, P_RZ };
-enum DiagOp { D_NEG, D_PHASE };
+enum DiagOp { D_NEG, D_PHASE, D_PHASE_INV };   // D_PHASE_INV: s with its sign flipped (the NP rotateZ)
 
 // Output i of a pair (r0.x, r0.y, r1.x, r1.y) takes mode (md >> 2i) & 3;
 // Hadamard's sums run on the integer pipes for any mode but MD_F.  `md`
@@ -194,6 +197,105 @@ __device__ __forceinline__ void diag_update(cplx<T> &a, const Coef<T> &k, unsign
     }
 }
 
+// ---------------------------------------------------------------------------
+// Updates of easy operands (lean.cuh): products and divisions on the integer
+// pipes, one FP64 add per output.  Each returns whether it ran; when it did
+// not, the amplitudes are unchanged and the caller takes the general update.
+// The test is a vote of the warp, so a warp with a zero (or otherwise not
+// easy) operand runs the general update alone and never both.  Only a
+// quotient that lean_div could not decide is left to its own thread.
+//
+// Bound by the FP64 pipe (two operations per SM and clock) and the ALU pipe
+// together: 98 instructions per amplitude and gate against 150 with the
+// general split "PPPQ", 2 of them FP64 instead of 2.7.  Two rotateX gates of a
+// 26-qubit dense state in one sweep: 757 us with the general split, 570 us
+// with this; FP64 pipe 72% busy, ALU pipe 58%.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool warp_all(bool x) { return __all_sync(__activemask(), x); }
+
+__device__ __forceinline__ double lean_prod(const emu::LeanOp &a, const emu::LeanK &k)
+{
+    return emu::dfrom(emu::lean_mul(a, k));
+}
+
+template <int OP>
+__device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const Coef<double> &k)
+{
+    if constexpr (OP == P_H) {
+        const double s0 = __dadd_rn(a0.x, a1.x), s1 = __dadd_rn(a0.y, a1.y);
+        const double d0 = __dsub_rn(a0.x, a1.x), d1 = __dsub_rn(a0.y, a1.y);
+        const uint64_t b0 = emu::dbits(s0), b1 = emu::dbits(s1), b2 = emu::dbits(d0), b3 = emu::dbits(d1);
+        if (!warp_all(k.ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) &
+                                         emu::easy_range(b3)))
+            return false;
+        bool sure = true;
+        const uint64_t q0 = emu::lean_div(emu::lean_operand(b0), k.ld, sure);
+        const uint64_t q1 = emu::lean_div(emu::lean_operand(b1), k.ld, sure);
+        const uint64_t q2 = emu::lean_div(emu::lean_operand(b2), k.ld, sure);
+        const uint64_t q3 = emu::lean_div(emu::lean_operand(b3), k.ld, sure);
+        if (!sure) return false;
+        a0 = make_double2(emu::dfrom(q0), emu::dfrom(q1));
+        a1 = make_double2(emu::dfrom(q2), emu::dfrom(q3));
+        return true;
+    } else {
+        const uint64_t b0 = emu::dbits(a0.x), b1 = emu::dbits(a0.y), b2 = emu::dbits(a1.x), b3 = emu::dbits(a1.y);
+        if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(b0) & emu::easy_product(b1) &
+                                                              emu::easy_product(b2) & emu::easy_product(b3)))
+            return false;
+        const emu::LeanOp x0 = emu::lean_operand(b0), y0 = emu::lean_operand(b1);
+        const emu::LeanOp x1 = emu::lean_operand(b2), y1 = emu::lean_operand(b3);
+        // the outputs' terms in pair_update's order
+        if constexpr (OP == P_RX) {
+            a0.x = __dadd_rn(lean_prod(x0, k.lc), lean_prod(y1, k.ls));
+            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(x1, k.ls));
+            a1.x = __dadd_rn(lean_prod(x1, k.lc), lean_prod(y0, k.ls));
+            a1.y = __dsub_rn(lean_prod(y1, k.lc), lean_prod(x0, k.ls));
+        } else if constexpr (OP == P_RY) {
+            a0.x = __dsub_rn(lean_prod(x0, k.lc), lean_prod(x1, k.ls));
+            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(y1, k.ls));
+            a1.x = __dadd_rn(lean_prod(x0, k.ls), lean_prod(x1, k.lc));
+            a1.y = __dadd_rn(lean_prod(y0, k.ls), lean_prod(y1, k.lc));
+        } else {
+            a0.x = __dadd_rn(lean_prod(x0, k.lc), lean_prod(y0, k.ls));
+            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(x0, k.ls));
+            a1.x = __dsub_rn(lean_prod(x1, k.lc), lean_prod(y1, k.ls));
+            a1.y = __dadd_rn(lean_prod(y1, k.lc), lean_prod(x1, k.ls));
+        }
+        return true;
+    }
+}
+
+template <int OP>
+__device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
+{
+    const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y);
+    if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
+    const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
+    const double xc = lean_prod(x, k.lc), ys = lean_prod(y, k.ls), yc = lean_prod(y, k.lc), xs = lean_prod(x, k.ls);
+    a.x = OP == D_PHASE ? __dsub_rn(xc, ys) : __dadd_rn(xc, ys);
+    a.y = OP == D_PHASE ? __dadd_rn(yc, xs) : __dsub_rn(yc, xs);
+    return true;
+}
+
+// A gate's update of a pair or of one amplitude: the easy form where it runs,
+// else the general one in modes `md`.
+template <class T, int OP, bool LEAN = true>
+__device__ __forceinline__ void pair_gate(cplx<T> &a0, cplx<T> &a1, const Coef<T> &k, unsigned md = 0)
+{
+    if constexpr (LEAN && sizeof(T) == 8 && OP != P_SWAP && OP != P_Y) {
+        if (pair_lean<OP>(a0, a1, k)) return;
+    }
+    pair_update<T, OP>(a0, a1, k, md);
+}
+template <class T, int OP, bool LEAN = true>
+__device__ __forceinline__ void diag_gate(cplx<T> &a, const Coef<T> &k, unsigned md = 0)
+{
+    if constexpr (LEAN && sizeof(T) == 8 && OP == D_PHASE) {
+        if (phase_lean<D_PHASE>(a, k)) return;
+    }
+    diag_update<T, OP>(a, k, md);
+}
+
 // The old single-bit masks (bit i set: output i fully on the integer pipes)
 // as a mode mask.
 __host__ __device__ constexpr unsigned modes_from_bits(unsigned em)
@@ -225,6 +327,24 @@ __host__ __device__ __forceinline__ IX ins00(IX j, unsigned lo, unsigned hi)
 #define QSLC_ITEMS 3
 #endif
 constexpr int ITEMS = QSLC_ITEMS;
+// The easy form (PAT_LEAN) has its own shape: items per iteration for pair
+// gates, Hadamard and diagonal gates, and CTAs of 256 threads per SM.
+// Measured on a dense 28-qubit state, TB/s of algorithmic bytes, rotateX /
+// phase: 1 item 6.12 / 5.23, 2 items 6.62 / 5.56, 3 items 6.53 / 5.79, 4
+// items - / 6.11 (four CTAs); rotateX with 2 items 6.25 on three CTAs and
+// 6.43 on five.  Hadamard ran 6.34 with one item and 4.09 with two.
+#ifndef QSLC_LEAN_ITEMS
+#define QSLC_LEAN_ITEMS 2
+#endif
+#ifndef QSLC_LEAN_ITEMS_H
+#define QSLC_LEAN_ITEMS_H 1
+#endif
+#ifndef QSLC_LEAN_ITEMS_D
+#define QSLC_LEAN_ITEMS_D 4
+#endif
+#ifndef QSLC_LEAN_CTAS
+#define QSLC_LEAN_CTAS 4
+#endif
 
 // Launch bounds of the sweep kernels: 256 threads, and with QSLC_MINB set,
 // at least that many resident CTAs per SM (which caps the registers).
@@ -233,40 +353,51 @@ constexpr int ITEMS = QSLC_ITEMS;
 #else
 #define QSLC_SWEEP_BOUNDS __launch_bounds__(256)
 #endif
+#define QSLC_LEAN_BOUNDS(CPAT) __launch_bounds__(256, (CPAT) == PAT_LEAN ? QSLC_LEAN_CTAS : 1)
 
-// A kernel's pattern is a template argument when it is one of the few
-// compiled in (the mask tests then fold away, and so do the unused
-// arithmetic paths and their registers); PAT_RUNTIME takes it from the
-// kernel's argument instead, for any other setting.
+// A kernel's pattern is a template argument where it is compiled in (the
+// mask tests then fold away, and so do the unused arithmetic paths and
+// their registers): 0, all on the FP64 pipe, and PAT_LEAN.  PAT_RUNTIME
+// takes it from the kernel's argument instead, for any other setting.
 constexpr unsigned PAT_RUNTIME = 0xFFFFFFFFu;
 
-// The patterns compiled in: the defaults below and their neighbours, so a
-// tuning sweep near the default measures compiled code too.  A pattern
-// holds one 8-bit mode mask per sweep item (item r at bits 8r..8r+7), 2 bits
-// per output (OutMode): e.g. 0x95 is P, P, P, Q for r0.x, r0.y, r1.x, r1.y,
-// and 0x9 is P, Q for a diagonal update's x, y.
-#ifndef QSLC_ROT_PATTERNS
-#define QSLC_ROT_PATTERNS 0u, 0x959595u, 0xA59595u, 0x159595u, 0x999999u, 0x969696u, 0x151515u, 0xA5A5A5u, 0x033333u
-#endif
-#ifndef QSLC_ROT2_PATTERNS
-#define QSLC_ROT2_PATTERNS 0u, 0x159595u, 0x959595u
-#endif
-#define QSLC_H_PATTERNS 0u, 0x000003u, 0x000303u
-#ifndef QSLC_DIAG_PATTERNS
-#define QSLC_DIAG_PATTERNS 0u, 0x090909u, 0x060606u, 0x010909u, 0x050909u, 0x030303u
-#endif
-#define QSLC_NP_PAIR_PATTERNS 0u, 0x030333u, 0x555555u, 0x959595u, 0xA5A5A5u
-#define QSLC_NP_DIAG_PATTERNS 0u, 0x000303u, 0x050505u, 0x090909u, 0x0A0A0Au
+// PAT_LEAN, the default of the complex128 sweeps: the easy form first
+// (pair_gate, diag_gate), with the default pattern for the warps it leaves.
+constexpr unsigned PAT_LEAN = 0xFFFFFFFEu;
 
-// Launch `f(std::integral_constant<unsigned, P>{})` with P = pat when pat is
-// one of CANDIDATES, else with PAT_RUNTIME.
-template <unsigned... CANDIDATES, class F>
-void with_pattern(unsigned pat, F &&f)
+// The default splits of the general path.  A pattern holds one 8-bit mode
+// mask per sweep item (item r at bits 8r..8r+7), 2 bits per output
+// (OutMode): 0x95 is P, P, P, Q for r0.x, r0.y, r1.x, r1.y, and 0x9 is P, Q
+// for a diagonal update's x, y.
+constexpr unsigned PAT_ROT = 0x959595u;
+constexpr unsigned PAT_H = 0u;
+constexpr unsigned PAT_DIAG = 0x090909u;
+
+// The mask of item r (the pattern repeats after three) of a sweep compiled
+// for CPAT, its general path in pattern DFLT when CPAT is PAT_LEAN.
+template <unsigned CPAT, unsigned DFLT>
+__device__ __forceinline__ unsigned item_modes(unsigned pat, int r)
 {
-    bool done = false;
-    ((pat == CANDIDATES && !done ? (f(std::integral_constant<unsigned, CANDIDATES>{}), done = true) : false),
-     ...);
-    if (!done) f(std::integral_constant<unsigned, PAT_RUNTIME>{});
+    const unsigned p = CPAT == PAT_RUNTIME ? pat : CPAT == PAT_LEAN ? DFLT : CPAT;
+    return (p >> (8 * (r % 3))) & 0xFFu;
+}
+template <int OP>
+constexpr unsigned pair_pattern() { return OP == P_H ? PAT_H : PAT_ROT; }
+
+template <unsigned CPAT, int LEAN_ITEMS>
+constexpr int sweep_items() { return CPAT == PAT_LEAN ? LEAN_ITEMS : ITEMS; }
+constexpr int pair_items(int op) { return op == P_H ? QSLC_LEAN_ITEMS_H : QSLC_LEAN_ITEMS; }
+
+// Launch `f(std::integral_constant<unsigned, P>{})` with P = PAT_LEAN when
+// `lean`, else 0 when pat is 0 (all on the FP64 pipe), else PAT_RUNTIME.
+// CHOICE is false where there is no arithmetic to place: P is 0 then.
+template <bool CHOICE, class F>
+void with_pattern(bool lean, unsigned pat, F &&f)
+{
+    if constexpr (!CHOICE) f(std::integral_constant<unsigned, 0u>{});
+    else if (lean) f(std::integral_constant<unsigned, PAT_LEAN>{});
+    else if (pat == 0) f(std::integral_constant<unsigned, 0u>{});
+    else f(std::integral_constant<unsigned, PAT_RUNTIME>{});
 }
 
 // Host-side coefficients, computed exactly as the reference does: in Fp,
@@ -283,6 +414,9 @@ Coef<T> coef(T c, T s)
     k.mc = emu::make_mulk(double(c));
     k.ms = emu::make_mulk(double(s));
     k.kd = emu::make_div(double(c));
+    k.lc = emu::make_lean(double(c));
+    k.ls = emu::make_lean(double(s));
+    k.ld = emu::make_lean_div(double(c));
     return k;
 }
 // The pattern a gate with coefficients k runs: `pat`, unless a coefficient
@@ -314,9 +448,9 @@ Coef<T> sqrt2_coef()
 }
 
 // Share of the dense updates' work done on the integer pipes, as a pattern
-// of one mode mask per sweep item (see ITEMS and OutMode).  The defaults
-// balance the FP64 pipe against the integer pipes on GB300; environment
-// variables override them for tuning: QSLC_EMU_MASK (rotations, one-qubit
+// of one mode mask per sweep item (see ITEMS and OutMode), where the easy
+// form does not run.  The environment variables that override the defaults
+// also turn the easy form off: QSLC_EMU_MASK (rotations, one-qubit
 // and controlled), QSLC_EMU_MASK_H (Hadamard), QSLC_EMU_MASK_DIAG (phase and
 // controlPhase), QSLC_EMU_MASK_NP and QSLC_EMU_MASK_NP_DIAG (the
 // number-preserving sweeps).  The value is one item ("PPPQ") or three
@@ -376,8 +510,39 @@ inline unsigned parse_pattern(const char *var, const char *dflt, unsigned output
 }
 inline unsigned pattern_rot()
 {
-    static unsigned p = parse_pattern("QSLC_EMU_MASK", "PPPQ,PPPQ,PPPF", 4);
+    static unsigned p = parse_pattern("QSLC_EMU_MASK", "PPPQ", 4);
     return p;
+}
+// Whether the variable is unset: the sweeps then run PAT_LEAN.
+inline bool unset(const char *var)
+{
+    const char *e = std::getenv(var);
+    return !(e && *e);
+}
+inline bool lean_rot()
+{
+    static const bool b = unset("QSLC_EMU_MASK");
+    return b;
+}
+inline bool lean_h()
+{
+    static const bool b = unset("QSLC_EMU_MASK_H");
+    return b;
+}
+inline bool lean_diag()
+{
+    static const bool b = unset("QSLC_EMU_MASK_DIAG");
+    return b;
+}
+inline bool lean_np_pair()
+{
+    static const bool b = unset("QSLC_EMU_MASK_NP");
+    return b;
+}
+inline bool lean_np_diag()
+{
+    static const bool b = unset("QSLC_EMU_MASK_NP_DIAG");
+    return b;
 }
 inline unsigned pattern_h()
 {
@@ -386,7 +551,7 @@ inline unsigned pattern_h()
 }
 inline unsigned pattern_diag()
 {
-    static unsigned p = parse_pattern("QSLC_EMU_MASK_DIAG", "PQ,PQ,PP", 2);
+    static unsigned p = parse_pattern("QSLC_EMU_MASK_DIAG", "PQ", 2);
     return p;
 }
 // The number-preserving sweeps spend integer work on ranking their indices,

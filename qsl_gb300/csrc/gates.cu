@@ -15,7 +15,8 @@
 //
 // Arithmetic is the reference's, operation for operation, with no
 // contraction into FMA: the x86-64 reference rounds each product and each
-// sum, and so does every update below (rn<T>::mul/add/sub/div).
+// sum, and so does every update below (rn<T>::mul/add/sub/div, and for
+// complex128 the integer forms of the same operations, gatemath.cuh).
 #include "qslc_internal.cuh"
 #include "gatemath.cuh"
 #include "stage.cuh"
@@ -53,17 +54,17 @@ __device__ __forceinline__ bool in_state(uint64_t i, uint64_t dim)
 
 // One-qubit pair gates: pairs (i0, i0 + 2^t), i0 = insert0(j, t).
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
-__global__ void QSLC_SWEEP_BOUNDS k_pair1(cplx<T> *__restrict__ st, uint64_t npairs,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair1(cplx<T> *__restrict__ st, uint64_t npairs,
                                                unsigned t, Coef<T> k, unsigned pat)
 {
+    constexpr int N = sweep_items<CPAT, pair_items(OP)>();
     const IX bit = IX(1) << t;
     const IX stride = IX(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
-    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(npairs); j += ITEMS * stride) {
-        cplx<T> a0[ITEMS], a1[ITEMS];
-        IX i0[ITEMS];
+    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(npairs); j += N * stride) {
+        cplx<T> a0[N], a1[N];
+        IX i0[N];
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             i0[r] = ins0<IX>(j + r * stride, t);
             if (j + r * stride < npairs && QSLC_IN_STATE(i0[r] | bit, 2 * npairs)) {
                 a0[r] = st[i0[r]];
@@ -71,9 +72,9 @@ __global__ void QSLC_SWEEP_BOUNDS k_pair1(cplx<T> *__restrict__ st, uint64_t npa
             }
         }
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             if (j + r * stride < npairs && QSLC_IN_STATE_QUIET(i0[r] | bit, 2 * npairs)) {
-                pair_update<T, OP>(a0[r], a1[r], k, (pt >> (8 * r)) & 0xFFu);
+                pair_gate<T, OP, CPAT == PAT_LEAN>(a0[r], a1[r], k, item_modes<CPAT, pair_pattern<OP>()>(pat, r));
                 st[i0[r]] = a0[r];
                 st[i0[r] | bit] = a1[r];
             }
@@ -184,24 +185,24 @@ __global__ void QSLC_SWEEP_BOUNDS k_pair1_shfl(cplx<T> *__restrict__ st, uint64_
 
 // One-qubit diagonal gates on the |1> half: index insert0(j, t) | 2^t.
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
-__global__ void QSLC_SWEEP_BOUNDS k_diag1(cplx<T> *__restrict__ st, uint64_t count,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_diag1(cplx<T> *__restrict__ st, uint64_t count,
                                                unsigned t, Coef<T> k, unsigned pat)
 {
+    constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS_D>();
     const IX bit = IX(1) << t;
     const IX stride = IX(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
-    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(count); j += ITEMS * stride) {
-        cplx<T> a[ITEMS];
-        IX i[ITEMS];
+    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(count); j += N * stride) {
+        cplx<T> a[N];
+        IX i[N];
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             i[r] = ins0<IX>(j + r * stride, t) | bit;
             if (j + r * stride < count && QSLC_IN_STATE(i[r], 2 * count)) a[r] = st[i[r]];
         }
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             if (j + r * stride < count && QSLC_IN_STATE_QUIET(i[r], 2 * count)) {
-                diag_update<T, OP>(a[r], k, (pt >> (8 * r)) & 0xFFu);
+                diag_gate<T, OP, CPAT == PAT_LEAN>(a[r], k, item_modes<CPAT, PAT_DIAG>(pat, r));
                 st[i[r]] = a[r];
             }
         }
@@ -248,36 +249,36 @@ __device__ __forceinline__ void group_apply(int op, cplx<T> &x0, cplx<T> &x1, cp
     constexpr unsigned D0 = QSLC_GROUP_MODES_DIAG & 0xFFu, D1 = (QSLC_GROUP_MODES_DIAG >> 8) & 0xFFu;
     switch (op) {
     case P_SWAP:
-        pair_update<T, P_SWAP>(x0, x1, k);
-        pair_update<T, P_SWAP>(y0, y1, k);
+        pair_gate<T, P_SWAP>(x0, x1, k);
+        pair_gate<T, P_SWAP>(y0, y1, k);
         break;
     case P_Y:
-        pair_update<T, P_Y>(x0, x1, k);
-        pair_update<T, P_Y>(y0, y1, k);
+        pair_gate<T, P_Y>(x0, x1, k);
+        pair_gate<T, P_Y>(y0, y1, k);
         break;
     case P_H:
-        pair_update<T, P_H>(x0, x1, k, H0);
-        pair_update<T, P_H>(y0, y1, k, H1);
+        pair_gate<T, P_H>(x0, x1, k, H0);
+        pair_gate<T, P_H>(y0, y1, k, H1);
         break;
     case P_RX:
-        pair_update<T, P_RX>(x0, x1, k, R0);
-        pair_update<T, P_RX>(y0, y1, k, R1);
+        pair_gate<T, P_RX>(x0, x1, k, R0);
+        pair_gate<T, P_RX>(y0, y1, k, R1);
         break;
     case P_RY:
-        pair_update<T, P_RY>(x0, x1, k, R0);
-        pair_update<T, P_RY>(y0, y1, k, R1);
+        pair_gate<T, P_RY>(x0, x1, k, R0);
+        pair_gate<T, P_RY>(y0, y1, k, R1);
         break;
     case P_RZ:
-        pair_update<T, P_RZ>(x0, x1, k, R0);
-        pair_update<T, P_RZ>(y0, y1, k, R1);
+        pair_gate<T, P_RZ>(x0, x1, k, R0);
+        pair_gate<T, P_RZ>(y0, y1, k, R1);
         break;
     case GROUP_DIAG + D_NEG:
-        diag_update<T, D_NEG>(x1, k);
-        diag_update<T, D_NEG>(y1, k);
+        diag_gate<T, D_NEG>(x1, k);
+        diag_gate<T, D_NEG>(y1, k);
         break;
     default:                                  // GROUP_DIAG + D_PHASE
-        diag_update<T, D_PHASE>(x1, k, D0);
-        diag_update<T, D_PHASE>(y1, k, D1);
+        diag_gate<T, D_PHASE>(x1, k, D0);
+        diag_gate<T, D_PHASE>(y1, k, D1);
         break;
     }
 }
@@ -285,8 +286,8 @@ __device__ __forceinline__ void group_apply(int op, cplx<T> &x0, cplx<T> &x1, cp
 // quads j in [0, 2^(n-2)): x = j with zeros inserted at bits lo < hi; the
 // first gate acts on bit mask c0, the second on c1 ({c0, c1} = {2^lo, 2^hi}).
 template <class T, class IX = uint64_t>
-__global__ void QSLC_SWEEP_BOUNDS k_group2(cplx<T> *__restrict__ st, uint64_t nquads, unsigned lo, unsigned hi,
-                                                IX c0, IX c1, GroupGates<T> g)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? QSLC_LEAN_CTAS : 1)
+    k_group2(cplx<T> *__restrict__ st, uint64_t nquads, unsigned lo, unsigned hi, IX c0, IX c1, GroupGates<T> g)
 {
     const IX stride = IX(gridDim.x) * blockDim.x;
     for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += stride) {
@@ -310,17 +311,17 @@ __global__ void QSLC_SWEEP_BOUNDS k_group2(cplx<T> *__restrict__ st, uint64_t nq
 // MODE 1: number-preserving pair (base|b1, base|b2);
 // MODE 2: fswap = MODE 1 swap plus negation of base|b1|b2.
 template <class T, int OP, int MODE, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
-__global__ void QSLC_SWEEP_BOUNDS k_pair2(cplx<T> *__restrict__ st, uint64_t nquads,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair2(cplx<T> *__restrict__ st, uint64_t nquads,
                                                unsigned lo, unsigned hi, uint64_t b1,
                                                uint64_t b2, Coef<T> k, unsigned pat)
 {
+    constexpr int N = sweep_items<CPAT, pair_items(OP)>();
     const IX stride = IX(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
-    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += ITEMS * stride) {
-        cplx<T> a0[ITEMS], a1[ITEMS];
-        IX x1[ITEMS], x2[ITEMS];
+    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += N * stride) {
+        cplx<T> a0[N], a1[N];
+        IX x1[N], x2[N];
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             const IX base = ins00<IX>(j + r * stride, lo, hi);
             x1[r] = base | IX(b1);
             x2[r] = (MODE == 0) ? (x1[r] | IX(b2)) : (base | IX(b2));
@@ -330,9 +331,9 @@ __global__ void QSLC_SWEEP_BOUNDS k_pair2(cplx<T> *__restrict__ st, uint64_t nqu
             }
         }
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             if (j + r * stride < nquads && QSLC_IN_STATE_QUIET(x1[r] | IX(b2), 4 * nquads)) {
-                pair_update<T, OP>(a0[r], a1[r], k, (pt >> (8 * r)) & 0xFFu);
+                pair_gate<T, OP, CPAT == PAT_LEAN>(a0[r], a1[r], k, item_modes<CPAT, pair_pattern<OP>()>(pat, r));
                 st[x1[r]] = a0[r];
                 st[x2[r]] = a1[r];
                 if constexpr (MODE == 2) {
@@ -348,24 +349,24 @@ __global__ void QSLC_SWEEP_BOUNDS k_pair2(cplx<T> *__restrict__ st, uint64_t nqu
 
 // controlZ / controlPhase: the |11> quarter (gates.cpp:277-301, :436-465).
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
-__global__ void QSLC_SWEEP_BOUNDS k_diag2(cplx<T> *__restrict__ st, uint64_t nquads,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_diag2(cplx<T> *__restrict__ st, uint64_t nquads,
                                                unsigned lo, unsigned hi, uint64_t both,
                                                Coef<T> k, unsigned pat)
 {
+    constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS_D>();
     const IX stride = IX(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
-    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += ITEMS * stride) {
-        cplx<T> a[ITEMS];
-        IX i[ITEMS];
+    for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += N * stride) {
+        cplx<T> a[N];
+        IX i[N];
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             i[r] = ins00<IX>(j + r * stride, lo, hi) | IX(both);
             if (j + r * stride < nquads && QSLC_IN_STATE(i[r], 4 * nquads)) a[r] = st[i[r]];
         }
 #pragma unroll
-        for (int r = 0; r < ITEMS; r++) {
+        for (int r = 0; r < N; r++) {
             if (j + r * stride < nquads && QSLC_IN_STATE_QUIET(i[r], 4 * nquads)) {
-                diag_update<T, OP>(a[r], k, (pt >> (8 * r)) & 0xFFu);
+                diag_gate<T, OP, CPAT == PAT_LEAN>(a[r], k, item_modes<CPAT, PAT_DIAG>(pat, r));
                 st[i[r]] = a[r];
             }
         }
@@ -618,8 +619,8 @@ __global__ void k_set_one(cplx<T> *st, uint64_t pos)
 // The staged sweeps take complex128 states of up to 31 qubits (32-bit
 // indices) with at least one whole tile, when QSLC_BULK=1.  They are not
 // the default: on dense 28-qubit states the register sweeps run rotations
-// at 5.56-5.67 TB/s and phase at 5.36-5.38, the best staged shape (8 warps,
-// 2 buffers, 4 pairs per lane, 3 CTAs per SM) at 5.28-5.35 and 5.11.
+// at 6.47-6.63 TB/s and phase at 6.11, the best staged shape (8 warps, 2
+// buffers, 4 pairs per lane, 3 CTAs per SM) at 5.28-5.35 and 5.11.
 inline bool bulk_enabled()
 {
     static const bool on = [] {
@@ -634,7 +635,7 @@ inline bool bulk_enabled()
 // pauliY, which move amplitudes without arithmetic: on a dense 28-qubit
 // state they run at 6.64-6.67 TB/s there against 6.16-6.69 for the
 // register sweeps.  The rotations and Hadamard stay on the register sweeps
-// (5.43-5.82 TB/s against 4.89-5.30 exchanged), whose thread computes both
+// (5.84-6.63 TB/s against 4.89-5.30 exchanged), whose thread computes both
 // outputs of a pair from operands it decodes once.  QSLC_SHFL=1 sends every
 // pair gate on those targets through the exchange, QSLC_SHFL=0 none.
 inline int shfl_mode()
@@ -712,10 +713,13 @@ int gate1_t(qslc_state *s, int gate, unsigned t, double angle)
     const bool bulk = use_bulk<T>(s);
     const uint32_t ntiles = bulk ? uint32_t(half / BULK_PAIRS) : 0;
     int brc = QSLC_OK;
-    auto pair = [&](auto op, unsigned pat0, const Coef<T> &k, auto cands) {
+    auto pair = [&](auto op, bool lean, unsigned pat0, const Coef<T> &k) {
         constexpr int OP = decltype(op)::value;
         const unsigned pat = OP == P_H ? pat0 : pattern_for(k, pat0);
-        cands(pat, [&](auto c) {
+        constexpr bool arith = sizeof(T) == 8 && OP != P_SWAP && OP != P_Y;
+        lean = lean && (OP == P_H || pat != 0) && !bulk && !use_shfl(OP, t, s->n);
+        with_pattern<arith>(lean, pat, [&](auto c) {
+            if constexpr (decltype(c)::value != PAT_LEAN) {
             if (use_shfl(OP, t, s->n)) {
                 with_index(s->n, [&](auto ix) {
                     k_pair1_shfl<T, OP, decltype(c)::value, decltype(ix)>
@@ -729,21 +733,19 @@ int gate1_t(qslc_state *s, int gate, unsigned t, double angle)
                     return;
                 }
             }
+            }
             with_index(s->n, [&](auto ix) {
                 k_pair1<T, OP, decltype(c)::value, decltype(ix)><<<grid, 256, 0, str>>>(st, half, t, k, pat);
             });
         });
     };
-    auto rot_c = [](unsigned p, auto f) { with_pattern<QSLC_ROT_PATTERNS>(p, f); };
-    auto h_c = [](unsigned p, auto f) { with_pattern<QSLC_H_PATTERNS>(p, f); };
-    auto none = [](unsigned p, auto f) { with_pattern<0u>(p, f); };
     switch (gate) {
-    case QSLC_PAULI_X: pair(std::integral_constant<int, P_SWAP>{}, 0, Coef<T>{}, none); break;
-    case QSLC_PAULI_Y: pair(std::integral_constant<int, P_Y>{}, 0, Coef<T>{}, none); break;
-    case QSLC_HADAMARD: pair(std::integral_constant<int, P_H>{}, had, sqrt2_coef<T>(), h_c); break;
-    case QSLC_ROTATE_X: pair(std::integral_constant<int, P_RX>{}, rot, half_angle<T>(angle), rot_c); break;
-    case QSLC_ROTATE_Y: pair(std::integral_constant<int, P_RY>{}, rot, half_angle<T>(angle), rot_c); break;
-    case QSLC_ROTATE_Z: pair(std::integral_constant<int, P_RZ>{}, rot, half_angle<T>(angle), rot_c); break;
+    case QSLC_PAULI_X: pair(std::integral_constant<int, P_SWAP>{}, false, 0, Coef<T>{}); break;
+    case QSLC_PAULI_Y: pair(std::integral_constant<int, P_Y>{}, false, 0, Coef<T>{}); break;
+    case QSLC_HADAMARD: pair(std::integral_constant<int, P_H>{}, lean_h(), had, sqrt2_coef<T>()); break;
+    case QSLC_ROTATE_X: pair(std::integral_constant<int, P_RX>{}, lean_rot(), rot, half_angle<T>(angle)); break;
+    case QSLC_ROTATE_Y: pair(std::integral_constant<int, P_RY>{}, lean_rot(), rot, half_angle<T>(angle)); break;
+    case QSLC_ROTATE_Z: pair(std::integral_constant<int, P_RZ>{}, lean_rot(), rot, half_angle<T>(angle)); break;
     case QSLC_PAULI_Z:
         if constexpr (sizeof(T) == 8) {
             if (bulk) {
@@ -758,8 +760,8 @@ int gate1_t(qslc_state *s, int gate, unsigned t, double angle)
     case QSLC_PHASE: {
         const Coef<T> k = full_angle<T>(angle);
         const unsigned pd = pattern_for(k, dg);
-        with_pattern<QSLC_DIAG_PATTERNS>(pd, [&](auto c) {
-            if constexpr (sizeof(T) == 8) {
+        with_pattern<sizeof(T) == 8>(lean_diag() && pd != 0 && !bulk, pd, [&](auto c) {
+            if constexpr (sizeof(T) == 8 && decltype(c)::value != PAT_LEAN) {
                 if (bulk) {
                     brc = launch_bulk<T>(s, k_diag1_bulk<T, D_PHASE, decltype(c)::value>, ntiles, t, k, pd);
                     return;
@@ -791,44 +793,42 @@ int gate2_t(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle)
     const bool dp = sizeof(T) == 8;
     const unsigned rot = dp ? pattern_rot() : 0, had = dp ? pattern_h() : 0, dg = dp ? pattern_diag() : 0;
     // pair kernel with operation OP, mode MODE, pattern pat among candidates
-    auto pair = [&](auto op, auto mode, unsigned pat0, const Coef<T> &k, auto cands) {
+    auto pair = [&](auto op, auto mode, bool lean, unsigned pat0, const Coef<T> &k) {
         constexpr int OP = decltype(op)::value, MODE = decltype(mode)::value;
         const unsigned pat = OP == P_H ? pat0 : pattern_for(k, pat0);
-        cands(pat, [&](auto c) {
+        constexpr bool arith = sizeof(T) == 8 && OP != P_SWAP && OP != P_Y;
+        with_pattern<arith>(lean && (OP == P_H || pat != 0), pat, [&](auto c) {
             with_index(s->n, [&](auto ix) {
                 k_pair2<T, OP, MODE, decltype(c)::value, decltype(ix)><<<grid, 256, 0, str>>>(st, quads, lo, hi, b1, b2,
                                                                                             k, pat);
             });
         });
     };
-    auto rot_c = [](unsigned p, auto f) { with_pattern<QSLC_ROT2_PATTERNS>(p, f); };
-    auto h_c = [](unsigned p, auto f) { with_pattern<QSLC_H_PATTERNS>(p, f); };
-    auto none = [](unsigned p, auto f) { with_pattern<0u>(p, f); };
     using M0 = std::integral_constant<int, 0>;
     using M1 = std::integral_constant<int, 1>;
     using M2 = std::integral_constant<int, 2>;
     switch (gate) {
-    case QSLC_CONTROL_NOT: pair(std::integral_constant<int, P_SWAP>{}, M0{}, 0, Coef<T>{}, none); break;
-    case QSLC_CONTROL_Y: pair(std::integral_constant<int, P_Y>{}, M0{}, 0, Coef<T>{}, none); break;
+    case QSLC_CONTROL_NOT: pair(std::integral_constant<int, P_SWAP>{}, M0{}, false, 0, Coef<T>{}); break;
+    case QSLC_CONTROL_Y: pair(std::integral_constant<int, P_Y>{}, M0{}, false, 0, Coef<T>{}); break;
     case QSLC_CONTROL_ROTATE_X:
-        pair(std::integral_constant<int, P_RX>{}, M0{}, rot, half_angle<T>(angle), rot_c);
+        pair(std::integral_constant<int, P_RX>{}, M0{}, lean_rot(), rot, half_angle<T>(angle));
         break;
     case QSLC_CONTROL_ROTATE_Y:
-        pair(std::integral_constant<int, P_RY>{}, M0{}, rot, half_angle<T>(angle), rot_c);
+        pair(std::integral_constant<int, P_RY>{}, M0{}, lean_rot(), rot, half_angle<T>(angle));
         break;
     case QSLC_CONTROL_ROTATE_Z:
-        pair(std::integral_constant<int, P_RZ>{}, M0{}, rot, half_angle<T>(angle), rot_c);
+        pair(std::integral_constant<int, P_RZ>{}, M0{}, lean_rot(), rot, half_angle<T>(angle));
         break;
-    case QSLC_CONTROL_HADAMARD: pair(std::integral_constant<int, P_H>{}, M0{}, had, sqrt2_coef<T>(), h_c); break;
-    case QSLC_SWAP: pair(std::integral_constant<int, P_SWAP>{}, M1{}, 0, Coef<T>{}, none); break;
+    case QSLC_CONTROL_HADAMARD: pair(std::integral_constant<int, P_H>{}, M0{}, lean_h(), had, sqrt2_coef<T>()); break;
+    case QSLC_SWAP: pair(std::integral_constant<int, P_SWAP>{}, M1{}, false, 0, Coef<T>{}); break;
     case QSLC_NP_ROTATE_X:
-        pair(std::integral_constant<int, P_RX>{}, M1{}, rot, half_angle<T>(angle), rot_c);
+        pair(std::integral_constant<int, P_RX>{}, M1{}, lean_rot(), rot, half_angle<T>(angle));
         break;
     case QSLC_NP_ROTATE_Y:
-        pair(std::integral_constant<int, P_RY>{}, M1{}, rot, half_angle<T>(angle), rot_c);
+        pair(std::integral_constant<int, P_RY>{}, M1{}, lean_rot(), rot, half_angle<T>(angle));
         break;
-    case QSLC_NP_HADAMARD: pair(std::integral_constant<int, P_H>{}, M1{}, had, sqrt2_coef<T>(), h_c); break;
-    case QSLC_FSWAP: pair(std::integral_constant<int, P_SWAP>{}, M2{}, 0, Coef<T>{}, none); break;
+    case QSLC_NP_HADAMARD: pair(std::integral_constant<int, P_H>{}, M1{}, lean_h(), had, sqrt2_coef<T>()); break;
+    case QSLC_FSWAP: pair(std::integral_constant<int, P_SWAP>{}, M2{}, false, 0, Coef<T>{}); break;
     case QSLC_CONTROL_Z:
         with_index(s->n, [&](auto ix) {
             k_diag2<T, D_NEG, 0u, decltype(ix)><<<grid, 256, 0, str>>>(st, quads, lo, hi, b1 | b2, Coef<T>{}, 0);
@@ -837,7 +837,7 @@ int gate2_t(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle)
     case QSLC_CONTROL_PHASE: {
         const Coef<T> k = full_angle<T>(angle);
         const unsigned pd = pattern_for(k, dg);
-        with_pattern<QSLC_DIAG_PATTERNS>(pd, [&](auto c) {
+        with_pattern<sizeof(T) == 8>(lean_diag() && pd != 0, pd, [&](auto c) {
             with_index(s->n, [&](auto ix) {
                 k_diag2<T, D_PHASE, decltype(c)::value, decltype(ix)><<<grid, 256, 0, str>>>(st, quads, lo, hi, b1 | b2,
                                                                                          k, pd);

@@ -1,0 +1,200 @@
+// lean.cuh -- exact binary64 products and a division by a constant on the
+// integer pipes, for operands that need no special cases.
+//
+// dpemu.cuh's prod_pack takes any operand: it tests each one for zero and
+// for its range, and shifts every product into place after multiplying.
+// The forms here take only "easy" operands -- normal, exponent field 65 to
+// 2044, low significand word not zero -- and leave every other operand to
+// the caller, which tests them first (easy_bits) and sends the whole warp
+// through the general path when a lane has one that is not easy.  What the
+// restriction buys:
+//   - no zero handling, and no rounding ties: a product lies half-way
+//     between two doubles only when the operand's significand has at least
+//     32 trailing zeros (see make_lean), so the sticky bits are not needed;
+//   - the shift moves before the product: whether ma * mc reaches 2^105 is
+//     one compare of ma with a constant (ceil(2^105 / mc)), and it selects
+//     the constant's significand shifted by 9 or by 10.  The product of that
+//     with ma << 2 always has its leading bit at bit 116, so its 53 bits
+//     are whole words from bit 64 up and the rounding is a carry out of the
+//     word below;
+//   - that carry, the significand and the sign/exponent word then go
+//     together in one three-word add.
+#pragma once
+
+#include "dpemu.cuh"
+
+namespace qslc {
+namespace emu {
+
+// A multiplier fixed for a whole kernel.
+struct LeanK {
+    uint32_t h0, h1;      // mc << 9, when ma * mc >= 2^105
+    uint32_t l0, l1;      // mc << 10, when it is below
+    uint32_t t0, t1;      // the least ma << 2 with ma * mc >= 2^105
+    uint32_t kh, kl;      // sign of c, and (e(c) - 1 + top) << 20, to be added to the operand's sign/exponent word
+    int usable;
+};
+
+inline LeanK make_lean(double c)
+{
+    LeanK r{};
+    const MulK m = make_mulk(c);
+    const uint64_t mc = (dbits(c) & MANT) | HIDDEN;
+    // ma * mc is a tie only when its trailing zeros number 51 or 52: with
+    // fewer than 20 of them in mc, only for an ma with 32 or more
+    r.usable = m.usable && (mc & ((uint64_t(1) << 20) - 1)) != 0;
+    r.h0 = uint32_t(mc << 9);
+    r.h1 = uint32_t((mc << 9) >> 32);
+    r.l0 = uint32_t(mc << 10);
+    r.l1 = uint32_t((mc << 10) >> 32);
+    const unsigned __int128 one = 1;
+    const uint64_t t = uint64_t(((one << 105) + mc - 1) / mc) << 2;
+    r.t0 = uint32_t(t);
+    r.t1 = uint32_t(t >> 32);
+    r.kl = m.ehi + m.sign;
+    r.kh = r.kl + 0x00100000u;
+    return r;
+}
+
+// The parts of an easy operand that its products share.
+struct LeanOp {
+    uint32_t lo, hi;      // ma << 2
+    uint32_t se;          // sign and exponent field, in place
+};
+
+QSLC_HD uint32_t shl2_hi(uint32_t lo, uint32_t hi)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, 2);
+#else
+    return (hi << 2) | (lo >> 30);
+#endif
+}
+
+QSLC_HD uint32_t mulhi32(uint32_t a, uint32_t b)
+{
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return uint32_t((uint64_t(a) * b) >> 32);
+#endif
+}
+
+QSLC_HD LeanOp lean_operand(uint64_t a)
+{
+    const uint32_t ahi = uint32_t(a >> 32), alo = uint32_t(a);
+    LeanOp o;
+    o.lo = alo << 2;
+    o.hi = (shl2_hi(alo, ahi) & 0x003FFFFFu) | 0x00400000u;
+    o.se = ahi & 0xFFF00000u;
+    return o;
+}
+
+// Whether an operand is in the exponent range (the low significand word is
+// tested on its own, where it matters).
+QSLC_HD bool easy_range(uint64_t a)
+{
+    const uint32_t ahi = uint32_t(a >> 32);
+    return (ahi + ahi) - 2 * PACK_EF_LO20 <= 2 * PACK_EF_SPAN20 + 0x001FFFFFu;
+}
+QSLC_HD bool easy_product(uint64_t a) { return easy_range(a) & (uint32_t(a) != 0); }
+
+// (r2:r1:r0) + (k:s1:s0), the top two words: one carry chain.
+QSLC_HD uint64_t round96(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t s0, uint32_t s1, uint32_t k, uint32_t &rest)
+{
+#ifdef __CUDA_ARCH__
+    uint32_t lo, hi;
+    asm("add.cc.u32 %0, %3, %4;\n\t"
+        "addc.cc.u32 %1, %5, %6;\n\t"
+        "addc.u32 %2, %7, %8;"
+        : "=&r"(rest), "=&r"(lo), "=r"(hi)
+        : "r"(r0), "r"(s0), "r"(r1), "r"(s1), "r"(r2), "r"(k));
+    return (uint64_t(hi) << 32) | lo;
+#else
+    const uint64_t t0 = uint64_t(r0) + s0;
+    rest = uint32_t(t0);
+    const uint64_t t1 = uint64_t(r1) + s1 + (t0 >> 32);
+    return (uint64_t(uint32_t(r2 + k + uint32_t(t1 >> 32))) << 32) | uint32_t(t1);
+#endif
+}
+
+// RN(a * c), packed.
+QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c)
+{
+    const bool top = ((uint64_t(a.hi) << 32) | a.lo) >= ((uint64_t(c.t1) << 32) | c.t0);
+    const uint32_t c0 = top ? c.h0 : c.l0, c1 = top ? c.h1 : c.l1, k = (top ? c.kh : c.kl) + a.se;
+    // partial sums stay below 2^64: c1 < 2^31, a.hi < 2^23
+    const uint64_t mid = mulwide(a.hi, c0) + (mulwide(a.lo, c1) + 0x80000000u);
+    const uint64_t high = mulwide(a.hi, c1);
+    uint32_t rest;
+    return round96(uint32_t(mid), uint32_t(high), uint32_t(high >> 32), mulhi32(a.lo, c0), uint32_t(mid >> 32), k,
+                   rest);
+}
+
+// A divisor fixed for a whole kernel: the reciprocals 2^146 / my (for
+// mx >= my) and 2^147 / my (for mx < my), rounded down, as three words.
+struct LeanDiv {
+    uint32_t h0, h1, h2, l0, l1, l2;
+    uint32_t t0, t1;      // my << 2
+    uint32_t kh, kl;      // sign of y, and (-e(y) + 1022 + top) << 20 less the operand's bias
+    int usable;
+};
+
+inline LeanDiv make_lean_div(double y)
+{
+    LeanDiv r{};
+    const DivConst d = make_div(y);
+    const uint64_t my = d.m;
+    auto recip = [my](int bits, uint32_t *w) {      // floor(2^bits / my), 145 <= bits <= 159
+        unsigned __int128 rem = 0;
+        uint32_t q[5];
+        for (int i = 0; i < 5; i++) {
+            const uint32_t digit = (bits / 32 == 4 - i) ? uint32_t(1) << (bits % 32) : 0u;
+            const unsigned __int128 cur = (rem << 32) | digit;
+            q[i] = uint32_t(cur / my);
+            rem = cur % my;
+        }
+        w[0] = q[4];
+        w[1] = q[3];
+        w[2] = q[2];
+        return (q[0] | q[1]) == 0 && q[2] < 0x80000000u && q[3] < 0xFF000000u;   // see lean_div's bounds
+    };
+    uint32_t h[3], l[3];
+    const bool fits = recip(146, h) & recip(147, l);
+    r.h0 = h[0], r.h1 = h[1], r.h2 = h[2];
+    r.l0 = l[0], r.l1 = l[1], r.l2 = l[2];
+    r.t0 = uint32_t(my << 2);
+    r.t1 = uint32_t((my << 2) >> 32);
+    // quotient exponent field ef - e(y) - (mx < my), less one for the hidden bit
+    r.kh = (uint32_t(-d.e - 1) << 20) + uint32_t(d.sign >> 32);
+    r.kl = r.kh - 0x00100000u;
+    // exponent fields 65 to 2044 divide to normal quotients for |e(y)| <= 1
+    r.usable = d.usable && fits && d.e >= -1 && d.e <= 1;
+    return r;
+}
+
+// RN(x / y), packed, for an operand in the exponent range; `sure` is
+// cleared when the quotient's fraction is too close to one half to decide.
+// With R the reciprocal, A = mx << 2, the quotient significand is the part
+// of A * R from bit 96 up and the word below it decides the rounding.  The
+// sum leaves out A.lo * r0 and the low words of A.lo * r1 and A.hi * r0, so
+// the word is low by less than four units, and R's own rounding adds less
+// than one.
+QSLC_HD uint64_t lean_div(const LeanOp &a, const LeanDiv &y, bool &sure)
+{
+    const bool top = ((uint64_t(a.hi) << 32) | a.lo) >= ((uint64_t(y.t1) << 32) | y.t0);
+    const uint32_t r0 = top ? y.h0 : y.l0, r1 = top ? y.h1 : y.l1, r2 = top ? y.h2 : y.l2;
+    const uint32_t k = (top ? y.kh : y.kl) + a.se;
+    // r1 < 2^32 - 2^24 and a.hi < 2^23: the sum of the two high words fits
+    const uint32_t low = mulhi32(a.lo, r1) + mulhi32(a.hi, r0);
+    const uint64_t mid = mulwide(a.hi, r1) + (mulwide(a.lo, r2) + 0x80000000u);
+    const uint64_t high = mulwide(a.hi, r2);
+    uint32_t rest;
+    const uint64_t q =
+        round96(uint32_t(mid), uint32_t(high), uint32_t(high >> 32), low, uint32_t(mid >> 32), k, rest);
+    sure = sure & (rest + 8u > 8u);
+    return q;
+}
+
+}  // namespace emu
+}  // namespace qslc

@@ -120,7 +120,7 @@ enum NPKind {
 // :183-185, :229-231).  NP_ITEMS items per grid-stride iteration; `pat`
 // chooses per item how each of the two outputs is computed (gatemath.cuh).
 template <class T, int K, unsigned CPAT = PAT_RUNTIME>
-__global__ void QSLC_SWEEP_BOUNDS k_np_single(cplx<T> *__restrict__ st,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_np_single(cplx<T> *__restrict__ st,
                                                    const uint32_t *__restrict__ tab, uint64_t count,
                                                    const uint32_t *__restrict__ rt, unsigned t1,
                                                    unsigned t2, uint32_t addbits, Coef<T> k,
@@ -128,7 +128,6 @@ __global__ void QSLC_SWEEP_BOUNDS k_np_single(cplx<T> *__restrict__ st,
 {
     using R = rn<T>;
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
     // the pattern-table entries of the next iteration are read while this
     // iteration's amplitudes are in flight, so the two dependent DRAM reads
     // of an item (its pattern, then its amplitude) overlap across iterations
@@ -162,7 +161,14 @@ __global__ void QSLC_SWEEP_BOUNDS k_np_single(cplx<T> *__restrict__ st,
 #pragma unroll
         for (int r = 0; r < NP_ITEMS; r++) {
             if (j + r * stride >= count) continue;
-            const unsigned md = (pt >> (8 * r)) & 0xFFu;
+            const unsigned md = item_modes<CPAT, PAT_DIAG>(pat, r);
+            if constexpr (K != NP_NEG1 && K != NP_CZ && CPAT == PAT_LEAN && sizeof(T) == 8) {
+                constexpr int OP = K == NP_RZ0 || K == NP_CRZ01 ? D_PHASE_INV : D_PHASE;
+                if (phase_lean<OP>(a[r], k)) {
+                    st[slot[r]] = a[r];
+                    continue;
+                }
+            }
             const T re = a[r].x, im = a[r].y;
             if constexpr (K == NP_NEG1 || K == NP_CZ) {
                 a[r].x = R::mul(re, T(-1));
@@ -183,14 +189,13 @@ __global__ void QSLC_SWEEP_BOUNDS k_np_single(cplx<T> *__restrict__ st,
 
 // Pair updates over table {n-2, w-1} (np/gates.cpp:236-415).
 template <class T, int K, unsigned CPAT = PAT_RUNTIME>
-__global__ void QSLC_SWEEP_BOUNDS k_np_pair(cplx<T> *__restrict__ st,
+__global__ void QSLC_LEAN_BOUNDS(CPAT) k_np_pair(cplx<T> *__restrict__ st,
                                                  const uint32_t *__restrict__ tab, uint64_t count,
                                                  const uint32_t *__restrict__ rt, unsigned lo,
                                                  unsigned hi, uint32_t b1, uint32_t b2, Coef<T> k,
                                                  unsigned pat)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    const unsigned pt = CPAT == PAT_RUNTIME ? pat : CPAT;
     // next iteration's pattern-table entries read ahead, as in k_np_single
     const uint64_t j0 = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     uint32_t xn[NP_ITEMS];
@@ -219,31 +224,10 @@ __global__ void QSLC_SWEEP_BOUNDS k_np_pair(cplx<T> *__restrict__ st,
 #pragma unroll
         for (int r = 0; r < NP_ITEMS; r++) {
             if (j + r * stride >= count) continue;
-            const unsigned md = (pt >> (8 * r)) & 0xFFu;
-            const unsigned E0 = mode_of(md, 0), E1 = mode_of(md, 1), E2 = mode_of(md, 2), E3 = mode_of(md, 3);
-            const cplx<T> p = a0[r], q = a1[r];
-            cplx<T> r0, r1;
-            if constexpr (K == NP_SWAP) {
-                r0 = q;
-                r1 = p;
-            } else if constexpr (K == NP_RX) {       // :316-321
-                r0.x = dot2m<T, false>(E0, p.x, k.c, k.kc, k.mc, q.y, k.s, k.ks, k.ms);
-                r0.y = dot2m<T, true>(E1, p.y, k.c, k.kc, k.mc, q.x, k.s, k.ks, k.ms);
-                r1.x = dot2m<T, false>(E2, q.x, k.c, k.kc, k.mc, p.y, k.s, k.ks, k.ms);
-                r1.y = dot2m<T, true>(E3, q.y, k.c, k.kc, k.mc, p.x, k.s, k.ks, k.ms);
-            } else if constexpr (K == NP_RY) {       // :366-371
-                r0.x = dot2m<T, true>(E0, p.x, k.c, k.kc, k.mc, q.x, k.s, k.ks, k.ms);
-                r0.y = dot2m<T, true>(E1, p.y, k.c, k.kc, k.mc, q.y, k.s, k.ks, k.ms);
-                r1.x = dot2m<T, false>(E2, p.x, k.s, k.ks, k.ms, q.x, k.c, k.kc, k.mc);
-                r1.y = dot2m<T, false>(E3, p.y, k.s, k.ks, k.ms, q.y, k.c, k.kc, k.mc);
-            } else {                                 // NP_H, :409-412
-                r0.x = hdiv<T, false>(E0 != MD_F, p.x, q.x, k);
-                r0.y = hdiv<T, false>(E1 != MD_F, p.y, q.y, k);
-                r1.x = hdiv<T, true>(E2 != MD_F, p.x, q.x, k);
-                r1.y = hdiv<T, true>(E3 != MD_F, p.y, q.y, k);
-            }
-            st[s1[r]] = r0;
-            st[s2[r]] = r1;
+            constexpr int OP = K == NP_SWAP ? P_SWAP : K == NP_RX ? P_RX : K == NP_RY ? P_RY : P_H;
+            pair_gate<T, OP, CPAT == PAT_LEAN>(a0[r], a1[r], k, item_modes<CPAT, pair_pattern<OP>()>(pat, r));
+            st[s1[r]] = a0[r];
+            st[s2[r]] = a1[r];
         }
     }
 }
@@ -410,7 +394,7 @@ static int np_gate_t(qslc_state *s, int gate, unsigned q1, unsigned q2, double a
         if constexpr (KIND == NP_NEG1 || KIND == NP_CZ)
             go(std::integral_constant<unsigned, 0u>{});
         else
-            with_pattern<QSLC_NP_DIAG_PATTERNS>(pat, go);
+            with_pattern<sizeof(T) == 8>(lean_np_diag() && pat != 0, pat, go);
         s->launches++;
     };
     auto pair = [&](auto kind_tag, Coef<T> k) {
@@ -428,9 +412,9 @@ static int np_gate_t(qslc_state *s, int gate, unsigned q1, unsigned q2, double a
         if constexpr (KIND == NP_SWAP)
             go(std::integral_constant<unsigned, 0u>{});
         else if constexpr (KIND == NP_H)
-            with_pattern<QSLC_H_PATTERNS>(pat, go);
+            with_pattern<sizeof(T) == 8>(lean_h(), pat, go);
         else
-            with_pattern<QSLC_NP_PAIR_PATTERNS>(pat, go);
+            with_pattern<sizeof(T) == 8>(lean_np_pair() && pat != 0, pat, go);
         s->launches++;
     };
     const unsigned lo = q1 < q2 ? q1 : q2, hi = q1 < q2 ? q2 : q1;
