@@ -159,20 +159,11 @@ int check_handle(const qslc_state *s)
     return QSLC_OK;
 }
 
-// Launch the one-qubit gate held back for grouping, alone.
-int release_held(qslc_state *s)
-{
-    if (!s->has_held) return QSLC_OK;
-    s->has_held = false;
-    return launch_gate1(s, s->held.code, s->held.q1, s->held.angle);
-}
-
-// Apply held and queued gates (the gate held for grouping; the precision
-// form's queue) before the state is read, and report a staged sweep whose
+// Apply held and queued gates (the run held back; the precision form's queue) before the state is read, and report a staged sweep whose
 // barrier wait ran out since the last check.
 int flushed(qslc_state *s)
 {
-    int hrc = release_held(s);
+    int hrc = run_release(s);
     if (!hrc) hrc = debug_bounds_error();
     if (hrc) return hrc;
     if (!s->fuse_queue.empty()) {
@@ -406,7 +397,7 @@ int qslc_assign(qslc_state *dst, const qslc_state *src)
     rc = flushed(const_cast<qslc_state *>(src));
     if (rc) return rc;
     dst->fuse_queue.clear();                 // overwritten below
-    dst->has_held = false;
+    run_drop(dst);
     if (dst->resizable && dst->namps != src->namps) {
         rc = resize_capacity(dst, src->namps);
         if (rc) return rc;
@@ -455,7 +446,7 @@ int qslc_reset(qslc_state *s)
     int rc = check_handle(s);
     if (rc) return rc;
     s->fuse_queue.clear();
-    s->has_held = false;
+    run_drop(s);
     return launch_fill_basis(s, 0);
 }
 
@@ -478,7 +469,7 @@ int qslc_set_state(qslc_state *s, const void *amps, uint64_t n_amps)
     if (n_amps != dim)
         return fail(QSLC_ESIZE, "Cannot assign state vector from different number of qubits");
     s->fuse_queue.clear();
-    s->has_held = false;
+    run_drop(s);
     if (!s->np) {
         QSLC_CUDA(cudaMemcpyAsync(s->amps, amps, dim * s->amp_bytes(), cudaMemcpyHostToDevice, s->stream));
         QSLC_CUDA(cudaStreamSynchronize(s->stream));
@@ -519,7 +510,7 @@ int qslc_set_basis(qslc_state *s, uint64_t index)
     if (s->n < 64 && index >= (uint64_t(1) << s->n))
         return fail(QSLC_EINVAL, "basis index out of range");
     s->fuse_queue.clear();
-    s->has_held = false;
+    run_drop(s);
     if (!s->np) return launch_fill_basis(s, index);
     const unsigned w = unsigned(__builtin_popcountll(index));
     if (w != s->nones) {
@@ -547,19 +538,7 @@ int qslc_gate1(qslc_state *s, int gate, unsigned targ, double angle)
         s->fuse_queue.push_back(GateOp{gate, targ, targ, angle});
         return QSLC_OK;
     }
-    if (!grouping_enabled()) return launch_gate1(s, gate, targ, angle);
-    // one-qubit gates on different qubits run two to a sweep: hold this
-    // one until the next call, which either joins it or releases it
-    const GateOp g{gate, targ, targ, angle};
-    if (s->has_held) {
-        s->has_held = false;
-        if (s->held.q1 != targ) return launch_group2(s, s->held, g);
-        rc = launch_gate1(s, s->held.code, s->held.q1, s->held.angle);
-        if (rc) return rc;
-    }
-    s->held = g;
-    s->has_held = true;
-    return QSLC_OK;
+    return run_push(s, GateOp{gate, targ, targ, angle});
 }
 
 int qslc_gate2(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle)
@@ -582,9 +561,7 @@ int qslc_gate2(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle)
         s->fuse_queue.push_back(GateOp{gate, q1, q2, angle});
         return QSLC_OK;
     }
-    rc = release_held(s);
-    if (rc) return rc;
-    return launch_gate2(s, gate, q1, q2, angle);
+    return run_push(s, GateOp{gate, q1, q2, angle});
 }
 
 int qslc_prob(qslc_state *s, unsigned targ, unsigned outcome, double *out)

@@ -14,6 +14,7 @@
 #include "lean.cuh"
 
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <type_traits>
 
@@ -22,8 +23,8 @@ namespace qslc {
 template <class T>
 struct Coef {
     T c, s;  // cos/sin of angle/2 (rotations) or of angle (phase); sqrt2 for H
-    emu::MulConst kc, ks;   // c and s decoded for the full integer path (double only)
-    emu::MulK mc, ms;       // c and s decoded for the integer products of the mixed path
+    emu::MulK mc, ms;       // c and s decoded for the integer products of the mixed path (double only)
+    emu::MulConst kc, ks;   // c and s decoded for the full integer path
     emu::DivConst kd;       // c as a divisor (Hadamard)
     emu::LeanK lc, ls;      // c and s for easy operands (lean.cuh)
     emu::LeanDiv ld;        // c as a divisor of easy operands
@@ -222,8 +223,11 @@ template <int OP>
 __device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const Coef<double> &k)
 {
     if constexpr (OP == P_H) {
-        const double s0 = __dadd_rn(a0.x, a1.x), s1 = __dadd_rn(a0.y, a1.y);
-        const double d0 = __dsub_rn(a0.x, a1.x), d1 = __dsub_rn(a0.y, a1.y);
+        double s0 = __dadd_rn(a0.x, a1.x), s1 = __dadd_rn(a0.y, a1.y);
+        double d0 = __dsub_rn(a0.x, a1.x), d1 = __dsub_rn(a0.y, a1.y);
+        // opaque from here: the compiler would otherwise compute the sums a
+        // second time after the vote, and the FP64 pipe is what binds
+        asm volatile("" : "+d"(s0), "+d"(s1), "+d"(d0), "+d"(d1));
         const uint64_t b0 = emu::dbits(s0), b1 = emu::dbits(s1), b2 = emu::dbits(d0), b3 = emu::dbits(d1);
         if (!warp_all(k.ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) &
                                          emu::easy_range(b3)))
@@ -275,25 +279,6 @@ __device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
     a.x = OP == D_PHASE ? __dsub_rn(xc, ys) : __dadd_rn(xc, ys);
     a.y = OP == D_PHASE ? __dadd_rn(yc, xs) : __dsub_rn(yc, xs);
     return true;
-}
-
-// A gate's update of a pair or of one amplitude: the easy form where it runs,
-// else the general one in modes `md`.
-template <class T, int OP, bool LEAN = true>
-__device__ __forceinline__ void pair_gate(cplx<T> &a0, cplx<T> &a1, const Coef<T> &k, unsigned md = 0)
-{
-    if constexpr (LEAN && sizeof(T) == 8 && OP != P_SWAP && OP != P_Y) {
-        if (pair_lean<OP>(a0, a1, k)) return;
-    }
-    pair_update<T, OP>(a0, a1, k, md);
-}
-template <class T, int OP, bool LEAN = true>
-__device__ __forceinline__ void diag_gate(cplx<T> &a, const Coef<T> &k, unsigned md = 0)
-{
-    if constexpr (LEAN && sizeof(T) == 8 && OP == D_PHASE) {
-        if (phase_lean<D_PHASE>(a, k)) return;
-    }
-    diag_update<T, OP>(a, k, md);
 }
 
 // The old single-bit masks (bit i set: output i fully on the integer pipes)
@@ -372,6 +357,149 @@ constexpr unsigned PAT_LEAN = 0xFFFFFFFEu;
 constexpr unsigned PAT_ROT = 0x959595u;
 constexpr unsigned PAT_H = 0u;
 constexpr unsigned PAT_DIAG = 0x090909u;
+
+// The general update of the warps that the easy forms leave.  A warp whose operands are all +0 (most of a sparse
+// state) only needs the signs of its zeros, which follow from the signs of
+// the coefficients: a sum of two zeros is -0 when both are, a difference p - q
+// when p is -0 and q is +0.
+//
+// The sweeps of several gates call it out of line (pair_slow and the like):
+// inline, once per gate type and pair, it would double their code.  There the
+// coefficients go by address (of a kernel parameter): by value they would take
+// registers and stack of every thread.  The sweeps of one gate have it
+// inline, where it costs them less than the call's registers: measured at 26
+// qubits, controlRotateX 201 against 212 us.
+struct SlowCoef {          // the first members of a Coef<double>
+    double c, s;
+    emu::MulK mc, ms;
+};
+static_assert(offsetof(Coef<double>, ms) == offsetof(SlowCoef, ms), "SlowCoef heads Coef<double>");
+__device__ __forceinline__ const SlowCoef *slow_coef(const Coef<double> &k)
+{
+    return reinterpret_cast<const SlowCoef *>(&k);
+}
+__device__ __forceinline__ Coef<double> general_coef(const SlowCoef *q)
+{
+    Coef<double> k{};
+    k.c = q->c;
+    k.s = q->s;
+    k.mc = q->mc;
+    k.ms = q->ms;
+    return k;
+}
+__device__ __forceinline__ double zero_of(uint32_t sign)
+{
+    return __hiloint2double(int(sign & 0x80000000u), 0);
+}
+__device__ __forceinline__ bool plus_zero(const double2 &a)
+{
+    return (emu::dbits(a.x) | emu::dbits(a.y)) == 0;
+}
+
+struct Pair {
+    double2 a0, a1;
+};
+template <int OP>
+__device__ __forceinline__ Pair pair_general(double2 a0, double2 a1, const SlowCoef *q)
+{
+    const Coef<double> k = general_coef(q);
+    if (warp_all(plus_zero(a0) & plus_zero(a1))) {
+        const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
+        const double add = zero_of(c & s), sub = zero_of(c & ~s);
+        if constexpr (OP == P_RX) a0 = a1 = make_double2(add, sub);
+        else if constexpr (OP == P_RY) {
+            a0 = make_double2(sub, sub);
+            a1 = make_double2(add, add);
+        } else {
+            a0 = make_double2(add, sub);
+            a1 = make_double2(sub, add);
+        }
+    } else {
+        pair_update<double, OP>(a0, a1, k, PAT_ROT & 0xFFu);
+    }
+    return Pair{a0, a1};
+}
+__device__ __forceinline__ Pair hadamard_general(double2 a0, double2 a1, double r, const emu::DivConst *kd)
+{
+    Coef<double> k{};
+    k.c = r;
+    k.kd = *kd;
+    // +0 +- +0 is +0, and so is its quotient
+    if (!warp_all(plus_zero(a0) & plus_zero(a1))) pair_update<double, P_H>(a0, a1, k, PAT_H & 0xFFu);
+    return Pair{a0, a1};
+}
+// x c - y s, y c + x s (INV: s with its sign flipped)
+template <bool INV>
+__device__ __forceinline__ double2 phase_general(double2 a, const SlowCoef *q)
+{
+    const Coef<double> k = general_coef(q);
+    const double x = a.x, y = a.y;
+    if (warp_all(plus_zero(a))) {
+        const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
+        const double add = zero_of(c & s), sub = zero_of(c & ~s);
+        return INV ? make_double2(add, sub) : make_double2(sub, add);
+    }
+    a.x = dot2m<double, !INV>(PAT_DIAG & 3u, x, k.c, k.kc, k.mc, y, k.s, k.ks, k.ms);
+    a.y = dot2m<double, INV>((PAT_DIAG >> 2) & 3u, y, k.c, k.kc, k.mc, x, k.s, k.ks, k.ms);
+    return a;
+}
+
+template <int OP>
+__device__ __noinline__ Pair pair_slow(double2 a0, double2 a1, const SlowCoef *q)
+{
+    return pair_general<OP>(a0, a1, q);
+}
+static __device__ __noinline__ Pair hadamard_slow(double2 a0, double2 a1, double r, const emu::DivConst *kd)
+{
+    return hadamard_general(a0, a1, r, kd);
+}
+template <bool INV>
+__device__ __noinline__ double2 phase_slow(double2 a, const SlowCoef *q)
+{
+    return phase_general<INV>(a, q);
+}
+
+// A gate's update of a pair or of one amplitude: the easy form where it runs,
+// else the general one, out of line, with the coefficients at `q` (`kd` for
+// Hadamard).
+template <int OP>
+__device__ __forceinline__ void pair_either(double2 &a0, double2 &a1, const Coef<double> &k, const SlowCoef *q,
+                                            const emu::DivConst *kd)
+{
+    if (pair_lean<OP>(a0, a1, k)) return;
+    Pair r;
+    if constexpr (OP == P_H) r = hadamard_slow(a0, a1, k.c, kd);
+    else r = pair_slow<OP>(a0, a1, q);
+    a0 = r.a0;
+    a1 = r.a1;
+}
+
+// The same for the sweeps of one gate, whose coefficients are a kernel
+// parameter; with LEAN false (and for gates without arithmetic) the general
+// update alone, in modes `md`.
+template <class T, int OP, bool LEAN>
+__device__ __forceinline__ void pair_gate(cplx<T> &a0, cplx<T> &a1, const Coef<T> &k, unsigned md)
+{
+    if constexpr (LEAN && sizeof(T) == 8 && OP != P_SWAP && OP != P_Y) {
+        if (pair_lean<OP>(a0, a1, k)) return;
+        Pair r;
+        if constexpr (OP == P_H) r = hadamard_general(a0, a1, k.c, &k.kd);
+        else r = pair_general<OP>(a0, a1, slow_coef(k));
+        a0 = r.a0;
+        a1 = r.a1;
+    } else {
+        pair_update<T, OP>(a0, a1, k, md);
+    }
+}
+template <class T, int OP, bool LEAN>
+__device__ __forceinline__ void diag_gate(cplx<T> &a, const Coef<T> &k, unsigned md)
+{
+    if constexpr (LEAN && sizeof(T) == 8 && OP != D_NEG) {
+        if (!phase_lean<OP>(a, k)) a = phase_general<OP == D_PHASE_INV>(a, slow_coef(k));
+    } else {
+        diag_update<T, OP>(a, k, md);
+    }
+}
 
 // The mask of item r (the pattern repeats after three) of a sweep compiled
 // for CPAT, its general path in pattern DFLT when CPAT is PAT_LEAN.

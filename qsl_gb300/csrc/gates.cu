@@ -3,7 +3,8 @@
 // The sweeps: k_pair1 / k_diag1 / k_pair2 / k_diag2, one gate per sweep
 // from registers; k_group2, two one-qubit gates on different qubits in one
 // sweep; k_pair1_shfl, pairs inside a warp exchanged between lanes; and
-// the staged sweeps through shared memory (opt-in, stage.cuh).
+// the staged sweeps through shared memory (opt-in, stage.cuh).  Runs of more
+// gates in one sweep are run.cu's.
 //
 // One thread owns one amplitude pair (or one amplitude for the diagonal
 // gates) in a grid-stride loop.  The pair index j is turned into the basis
@@ -19,6 +20,7 @@
 // complex128 the integer forms of the same operations, gatemath.cuh).
 #include "qslc_internal.cuh"
 #include "gatemath.cuh"
+#include "gateops.cuh"
 #include "stage.cuh"
 
 #include <cmath>
@@ -55,7 +57,7 @@ __device__ __forceinline__ bool in_state(uint64_t i, uint64_t dim)
 // One-qubit pair gates: pairs (i0, i0 + 2^t), i0 = insert0(j, t).
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair1(cplx<T> *__restrict__ st, uint64_t npairs,
-                                               unsigned t, Coef<T> k, unsigned pat)
+                                               unsigned t, const __grid_constant__ Coef<T> k, unsigned pat)
 {
     constexpr int N = sweep_items<CPAT, pair_items(OP)>();
     const IX bit = IX(1) << t;
@@ -186,7 +188,7 @@ __global__ void QSLC_SWEEP_BOUNDS k_pair1_shfl(cplx<T> *__restrict__ st, uint64_
 // One-qubit diagonal gates on the |1> half: index insert0(j, t) | 2^t.
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_diag1(cplx<T> *__restrict__ st, uint64_t count,
-                                               unsigned t, Coef<T> k, unsigned pat)
+                                               unsigned t, const __grid_constant__ Coef<T> k, unsigned pat)
 {
     constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS_D>();
     const IX bit = IX(1) << t;
@@ -216,86 +218,29 @@ __global__ void QSLC_LEAN_BOUNDS(CPAT) k_diag1(cplx<T> *__restrict__ st, uint64_
 // amplitude sees the same operations, in the same order, as in two
 // sweeps, so the bits are those of the two gates one after the other; the
 // state is read and written once instead of twice.
-//
-// `op` is a PairOp, or GROUP_DIAG + a DiagOp for phase and pauliZ (which
-// act on the members with the bit set).  The output modes (gatemath.cuh)
-// are fixed per gate type: the two pair updates of a rotation take the
-// low and high byte of QSLC_GROUP_MODES_ROT, and so on.
-constexpr int GROUP_DIAG = 16;
-#ifndef QSLC_GROUP_MODES_ROT
-#define QSLC_GROUP_MODES_ROT 0x1595u      // PPPQ, PPPF
-#endif
-#ifndef QSLC_GROUP_MODES_H
-#define QSLC_GROUP_MODES_H 0x0000u        // FFFF, FFFF
-#endif
-#ifndef QSLC_GROUP_MODES_DIAG
-#define QSLC_GROUP_MODES_DIAG 0x0509u     // PQ, PP
-#endif
-
 template <class T>
 struct GroupGates {
     int op[2];
     Coef<T> k[2];
 };
 
-// One gate of a group on the pairs (x0, x1) and (y0, y1); x1 and y1 are
-// the members with the gate's bit set.
-template <class T>
-__device__ __forceinline__ void group_apply(int op, cplx<T> &x0, cplx<T> &x1, cplx<T> &y0, cplx<T> &y1,
-                                            const Coef<T> &k)
-{
-    constexpr unsigned R0 = QSLC_GROUP_MODES_ROT & 0xFFu, R1 = (QSLC_GROUP_MODES_ROT >> 8) & 0xFFu;
-    constexpr unsigned H0 = QSLC_GROUP_MODES_H & 0xFFu, H1 = (QSLC_GROUP_MODES_H >> 8) & 0xFFu;
-    constexpr unsigned D0 = QSLC_GROUP_MODES_DIAG & 0xFFu, D1 = (QSLC_GROUP_MODES_DIAG >> 8) & 0xFFu;
-    switch (op) {
-    case P_SWAP:
-        pair_gate<T, P_SWAP>(x0, x1, k);
-        pair_gate<T, P_SWAP>(y0, y1, k);
-        break;
-    case P_Y:
-        pair_gate<T, P_Y>(x0, x1, k);
-        pair_gate<T, P_Y>(y0, y1, k);
-        break;
-    case P_H:
-        pair_gate<T, P_H>(x0, x1, k, H0);
-        pair_gate<T, P_H>(y0, y1, k, H1);
-        break;
-    case P_RX:
-        pair_gate<T, P_RX>(x0, x1, k, R0);
-        pair_gate<T, P_RX>(y0, y1, k, R1);
-        break;
-    case P_RY:
-        pair_gate<T, P_RY>(x0, x1, k, R0);
-        pair_gate<T, P_RY>(y0, y1, k, R1);
-        break;
-    case P_RZ:
-        pair_gate<T, P_RZ>(x0, x1, k, R0);
-        pair_gate<T, P_RZ>(y0, y1, k, R1);
-        break;
-    case GROUP_DIAG + D_NEG:
-        diag_gate<T, D_NEG>(x1, k);
-        diag_gate<T, D_NEG>(y1, k);
-        break;
-    default:                                  // GROUP_DIAG + D_PHASE
-        diag_gate<T, D_PHASE>(x1, k, D0);
-        diag_gate<T, D_PHASE>(y1, k, D1);
-        break;
-    }
-}
-
 // quads j in [0, 2^(n-2)): x = j with zeros inserted at bits lo < hi; the
 // first gate acts on bit mask c0, the second on c1 ({c0, c1} = {2^lo, 2^hi}).
-template <class T, class IX = uint64_t>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? QSLC_LEAN_CTAS : 1)
-    k_group2(cplx<T> *__restrict__ st, uint64_t nquads, unsigned lo, unsigned hi, IX c0, IX c1, GroupGates<T> g)
+// ARITH false is the sweep of two gates that only move amplitudes or change
+// signs: without the arithmetic's registers and stack it runs at HBM speed
+// (two pauliX at 26 qubits: 330 us, with them 356).
+template <class T, class IX, bool ARITH>
+__global__ void __launch_bounds__(256, sizeof(T) == 8 && ARITH ? QSLC_LEAN_CTAS : 1)
+    k_group2(cplx<T> *__restrict__ st, uint64_t nquads, unsigned lo, unsigned hi, IX c0, IX c1,
+             const __grid_constant__ GroupGates<T> g)
 {
     const IX stride = IX(gridDim.x) * blockDim.x;
     for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += stride) {
         const IX x = ins00<IX>(j, lo, hi);
         if (!QSLC_IN_STATE(x | c0 | c1, 4 * nquads)) continue;
         cplx<T> a00 = st[x], a01 = st[x | c0], a10 = st[x | c1], a11 = st[x | c0 | c1];
-        group_apply<T>(g.op[0], a00, a01, a10, a11, g.k[0]);
-        group_apply<T>(g.op[1], a00, a10, a01, a11, g.k[1]);
+        group_apply<T, ARITH>(g.op[0], a00, a01, a10, a11, g.k[0]);
+        group_apply<T, ARITH>(g.op[1], a00, a10, a01, a11, g.k[1]);
         st[x] = a00;
         st[x | c0] = a01;
         st[x | c1] = a10;
@@ -313,7 +258,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 8 ? QSLC_LEAN_CTAS : 1)
 template <class T, int OP, int MODE, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair2(cplx<T> *__restrict__ st, uint64_t nquads,
                                                unsigned lo, unsigned hi, uint64_t b1,
-                                               uint64_t b2, Coef<T> k, unsigned pat)
+                                               uint64_t b2, const __grid_constant__ Coef<T> k, unsigned pat)
 {
     constexpr int N = sweep_items<CPAT, pair_items(OP)>();
     const IX stride = IX(gridDim.x) * blockDim.x;
@@ -351,7 +296,7 @@ __global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair2(cplx<T> *__restrict__ st, uint64_
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_diag2(cplx<T> *__restrict__ st, uint64_t nquads,
                                                unsigned lo, unsigned hi, uint64_t both,
-                                               Coef<T> k, unsigned pat)
+                                               const __grid_constant__ Coef<T> k, unsigned pat)
 {
     constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS_D>();
     const IX stride = IX(gridDim.x) * blockDim.x;
@@ -880,8 +825,13 @@ int group2_t(qslc_state *s, const GateOp &g0, const GateOp &g1)
     auto *st = static_cast<cplx<T> *>(s->amps);
     with_index(s->n, [&](auto ix) {
         using IX = decltype(ix);
-        k_group2<T, IX><<<grid_for(quads), 256, 0, s->stream>>>(st, quads, lo, hi, IX(1) << g0.q1,
-                                                               IX(1) << g1.q1, g);
+        auto moves = [](int op) { return op == P_SWAP || op == P_Y || op == GROUP_DIAG + D_NEG; };
+        if (moves(g.op[0]) && moves(g.op[1]))
+            k_group2<T, IX, false><<<grid_for(quads), 256, 0, s->stream>>>(st, quads, lo, hi, IX(1) << g0.q1,
+                                                                         IX(1) << g1.q1, g);
+        else
+            k_group2<T, IX, true><<<grid_for(quads), 256, 0, s->stream>>>(st, quads, lo, hi, IX(1) << g0.q1,
+                                                                        IX(1) << g1.q1, g);
     });
     s->launches++;
     QSLC_CUDA(cudaGetLastError());
@@ -890,14 +840,13 @@ int group2_t(qslc_state *s, const GateOp &g0, const GateOp &g1)
 
 }  // namespace
 
-// Grouping is on unless QSLC_GROUP=0.
-bool grouping_enabled()
+GroupMode group_mode()
 {
-    static const bool on = [] {
+    static const GroupMode m = [] {
         const char *e = std::getenv("QSLC_GROUP");
-        return !(e && e[0] == '0');
+        return !e || !*e ? GROUP_RUNS : e[0] == '0' ? GROUP_OFF : GROUP_PAIRS;
     }();
-    return on;
+    return m;
 }
 
 int launch_group2(qslc_state *s, const GateOp &g0, const GateOp &g1)

@@ -21,6 +21,8 @@
 //     together in one three-word add.
 #pragma once
 
+#include <cmath>
+
 #include "dpemu.cuh"
 
 namespace qslc {
@@ -194,6 +196,28 @@ QSLC_HD uint64_t lean_div(const LeanOp &a, const LeanDiv &y, bool &sure)
         round96(uint32_t(mid), uint32_t(high), uint32_t(high >> 32), low, uint32_t(mid >> 32), k, rest);
     sure = sure & (rest + 8u > 8u);
     return q;
+}
+
+// RN(x / d) in binary32 for a constant d, r = RN(1 / d), by Markstein's final
+// step (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): q within an ulp of the quotient, its exact
+// remainder, and one fused correction.  Zeros keep their sign in this
+// arrangement of the signs.  Takes zeros and magnitudes from 2^-100 up
+// (div_step_takes); the others go to the divide instruction sequence.
+QSLC_HD float div_step(float x, float d, float r)
+{
+#ifdef __CUDA_ARCH__
+    const float q = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(q, d, -x), -r, q);
+#else
+    volatile float q = x * r;
+    return std::fma(std::fma(float(q), d, -x), -r, float(q));
+#endif
+}
+QSLC_HD bool div_step_takes(float x)
+{
+    const float m = x < 0.f ? -x : x;
+    return m == 0.f || (m >= 0x1p-100f && m <= 0x1.fffffep127f);
 }
 
 }  // namespace emu

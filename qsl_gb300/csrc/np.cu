@@ -123,7 +123,7 @@ template <class T, int K, unsigned CPAT = PAT_RUNTIME>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_np_single(cplx<T> *__restrict__ st,
                                                    const uint32_t *__restrict__ tab, uint64_t count,
                                                    const uint32_t *__restrict__ rt, unsigned t1,
-                                                   unsigned t2, uint32_t addbits, Coef<T> k,
+                                                   unsigned t2, uint32_t addbits, const __grid_constant__ Coef<T> k,
                                                    unsigned pat)
 {
     using R = rn<T>;
@@ -163,11 +163,9 @@ __global__ void QSLC_LEAN_BOUNDS(CPAT) k_np_single(cplx<T> *__restrict__ st,
             if (j + r * stride >= count) continue;
             const unsigned md = item_modes<CPAT, PAT_DIAG>(pat, r);
             if constexpr (K != NP_NEG1 && K != NP_CZ && CPAT == PAT_LEAN && sizeof(T) == 8) {
-                constexpr int OP = K == NP_RZ0 || K == NP_CRZ01 ? D_PHASE_INV : D_PHASE;
-                if (phase_lean<OP>(a[r], k)) {
-                    st[slot[r]] = a[r];
-                    continue;
-                }
+                diag_gate<T, K == NP_RZ0 || K == NP_CRZ01 ? D_PHASE_INV : D_PHASE, true>(a[r], k, md);
+                st[slot[r]] = a[r];
+                continue;
             }
             const T re = a[r].x, im = a[r].y;
             if constexpr (K == NP_NEG1 || K == NP_CZ) {
@@ -192,7 +190,7 @@ template <class T, int K, unsigned CPAT = PAT_RUNTIME>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_np_pair(cplx<T> *__restrict__ st,
                                                  const uint32_t *__restrict__ tab, uint64_t count,
                                                  const uint32_t *__restrict__ rt, unsigned lo,
-                                                 unsigned hi, uint32_t b1, uint32_t b2, Coef<T> k,
+                                                 unsigned hi, uint32_t b1, uint32_t b2, const __grid_constant__ Coef<T> k,
                                                  unsigned pat)
 {
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;

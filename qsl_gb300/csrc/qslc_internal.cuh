@@ -140,10 +140,11 @@ struct qslc_state {
     qslc::Scratch fuse_mats;
     qslc::Scratch fuse_tc_mats;   // packed tensor-core operands, then an error word
     uint64_t fused_blocks = 0;
-    // a one-qubit gate held back to run in one sweep with the next
-    // one-qubit gate on another qubit (gates.cu, k_group2)
-    qslc::GateOp held{};
-    bool has_held = false;
+    // gates of a plain state held back to run in one sweep (run.cu), and
+    // the qubits they act on
+    std::vector<qslc::GateOp> run;
+    uint64_t run_mask = 0;
+    size_t run_ops = 0;
     int *wait_err = nullptr;         // device word set by a staged sweep whose barrier wait ran out
     bool wait_err_pending = false;   // staged sweeps launched since the word was last read
 
@@ -176,7 +177,10 @@ int launch_gate1(qslc_state *s, int gate, unsigned targ, double angle);
 int launch_gate2(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle);
 // two one-qubit gates on different qubits, in this order, in one sweep
 int launch_group2(qslc_state *s, const GateOp &g0, const GateOp &g1);
-bool grouping_enabled();
+// How gates on a plain state are held back (QSLC_GROUP): not at all ("0"),
+// one-qubit gates two to a sweep ("1"), or runs of any gates (unset).
+enum GroupMode { GROUP_OFF, GROUP_PAIRS, GROUP_RUNS };
+GroupMode group_mode();
 // Debug builds (-DQSLC_DEBUG_BOUNDS): QSLC_EINVAL when a sweep met an index
 // outside its state since the last call; QSLC_OK otherwise and in default
 // builds.
@@ -185,6 +189,11 @@ int launch_collapse(qslc_state *s, unsigned targ, unsigned outcome, double facto
 // complex64 collapse with the factor applied in double (precision form)
 int launch_collapse_f64(qslc_state *s, unsigned targ, unsigned outcome, double factor);
 int launch_fill_basis(qslc_state *s, uint64_t pos);
+
+// run.cu: hold a gate back, apply what is held, forget it
+int run_push(qslc_state *s, const GateOp &g);
+int run_release(qslc_state *s);
+void run_drop(qslc_state *s);
 
 // fused.cu
 int fusion_flush(qslc_state *s);
