@@ -265,11 +265,11 @@ QSLC_API uint64_t qslc_fused_blocks(const qslc_state *s);
  * nlayers[i] layers of: rotateY on every qubit, rotateZ on every qubit,
  * controlNot(q, q+1) for q = 0..n-2; then prob(q, 0) and prob(q, 1) for
  * every q and `nshots` sampleAll draws.  All instances run in one
- * persistent kernel, followed by one kernel that walks the sampling CDFs,
- * both captured once in a CUDA graph.  Results are the bits qsl's Default
+ * persistent kernel, with kernels for the probabilities and the shots after
+ * it, all captured once in a CUDA graph.  Results are the bits qsl's Default
  * backend gives for the same calls.  Device memory: the instances' inputs
- * and results, 8 bytes per amplitude of every instance (the |a|^2 terms
- * of the CDFs), and two state buffers per CTA of the largest instance
+ * and results, 8 (4 for QSLC_C64) bytes per amplitude of every instance (the |a|^2 terms
+ * of the CDFs), and two state buffers per cluster of CTAs of the largest instance
  * when it does not fit a shared-memory tile. */
 typedef struct qslc_batch qslc_batch;
 QSLC_API int qslc_batch_create(int dtype, uint32_t ninst, const uint32_t *nqubits,
@@ -277,9 +277,9 @@ QSLC_API int qslc_batch_create(int dtype, uint32_t ninst, const uint32_t *nqubit
 /* angles: per instance, layer-major, per qubit (rotateY angle, rotateZ
  * angle); uniforms: nshots per instance.  probs: per instance 2*n values
  * (prob(q,0), prob(q,1)), q ascending; shots: nshots per instance, in the
- * order of the uniforms.  The call's host work (coefficients, sorting each
- * instance's uniforms, reordering the shots) runs on up to 32 host threads
- * it starts and joins before it returns. */
+ * order of the uniforms.  The call's host work (coefficients, and above 4096
+ * shots an instance the sorting of its uniforms) runs on up to 32 host
+ * threads it starts and joins before it returns. */
 QSLC_API int qslc_batch_run(qslc_batch *b, const double *angles, const double *uniforms,
                             double *probs, uint64_t *shots);
 /* Measure every launch shape (threads per CTA, shared-memory tile of 64 or

@@ -281,6 +281,19 @@ __device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
     return true;
 }
 
+// x c - y s, y c + x s with s negated when `flip` is 0x80000000 (0 otherwise).
+__device__ __forceinline__ bool phase_flip_lean(double2 &a, uint32_t flip, const Coef<double> &k)
+{
+    const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y), f = uint64_t(flip) << 32;
+    if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
+    const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
+    const double xc = lean_prod(x, k.lc), ys = emu::dfrom(emu::lean_mul(y, k.ls) ^ f);
+    const double yc = lean_prod(y, k.lc), xs = emu::dfrom(emu::lean_mul(x, k.ls) ^ f);
+    a.x = __dsub_rn(xc, ys);
+    a.y = __dadd_rn(yc, xs);
+    return true;
+}
+
 // The old single-bit masks (bit i set: output i fully on the integer pipes)
 // as a mode mask.
 __host__ __device__ constexpr unsigned modes_from_bits(unsigned em)

@@ -28,16 +28,28 @@
 namespace qslc {
 namespace emu {
 
-// A multiplier fixed for a whole kernel.
-struct LeanK {
+// A multiplier fixed for a whole kernel: two 16-byte words.
+struct alignas(16) LeanK {
     uint32_t h0, h1;      // mc << 9, when ma * mc >= 2^105
     uint32_t l0, l1;      // mc << 10, when it is below
     uint32_t t0, t1;      // the least ma << 2 with ma * mc >= 2^105
-    uint32_t kh, kl;      // sign of c, and (e(c) - 1 + top) << 20, to be added to the operand's sign/exponent word
+    uint32_t k;           // sign of c and (e(c) - 1) << 20, to be added to the operand's sign/exponent word
     int usable;
 };
 
-inline LeanK make_lean(double c)
+// ceil(2^105 / m) for a significand m: the IEEE quotient is the nearest
+// integer to it, low by at most one.
+QSLC_HD uint64_t ceil_2_105(uint64_t m)
+{
+#ifdef __CUDA_ARCH__
+    uint64_t q = uint64_t(__ddiv_rn(0x1p105, double((long long)m)));
+#else
+    uint64_t q = uint64_t(0x1p105 / double(m));
+#endif
+    return umulhi(q, m) >= (uint64_t(1) << 41) ? q : q + 1;
+}
+
+QSLC_HD LeanK make_lean(double c)
 {
     LeanK r{};
     const MulK m = make_mulk(c);
@@ -49,12 +61,10 @@ inline LeanK make_lean(double c)
     r.h1 = uint32_t((mc << 9) >> 32);
     r.l0 = uint32_t(mc << 10);
     r.l1 = uint32_t((mc << 10) >> 32);
-    const unsigned __int128 one = 1;
-    const uint64_t t = uint64_t(((one << 105) + mc - 1) / mc) << 2;
+    const uint64_t t = ceil_2_105(mc) << 2;
     r.t0 = uint32_t(t);
     r.t1 = uint32_t(t >> 32);
-    r.kl = m.ehi + m.sign;
-    r.kh = r.kl + 0x00100000u;
+    r.k = m.ehi + m.sign;
     return r;
 }
 
@@ -124,7 +134,8 @@ QSLC_HD uint64_t round96(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t s0, uin
 QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c)
 {
     const bool top = ((uint64_t(a.hi) << 32) | a.lo) >= ((uint64_t(c.t1) << 32) | c.t0);
-    const uint32_t c0 = top ? c.h0 : c.l0, c1 = top ? c.h1 : c.l1, k = (top ? c.kh : c.kl) + a.se;
+    const uint32_t c0 = top ? c.h0 : c.l0, c1 = top ? c.h1 : c.l1;
+    const uint32_t k = c.k + a.se + (top ? 0x00100000u : 0u);
     // partial sums stay below 2^64: c1 < 2^31, a.hi < 2^23
     const uint64_t mid = mulwide(a.hi, c0) + (mulwide(a.lo, c1) + 0x80000000u);
     const uint64_t high = mulwide(a.hi, c1);

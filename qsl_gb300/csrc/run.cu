@@ -119,17 +119,7 @@ __device__ __forceinline__ void run_pairs(double2 &x0, double2 &x1, double2 &y0,
 
 __device__ __forceinline__ void run_rotate(double2 &a, uint32_t flip, const Coef<double> &k, const SlowCoef *q)
 {
-    const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y);
-    const uint64_t f = uint64_t(flip) << 32;
-    if (warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) {
-        const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
-        const double xc = lean_prod(x, k.lc), ys = emu::dfrom(emu::lean_mul(y, k.ls) ^ f);
-        const double yc = lean_prod(y, k.lc), xs = emu::dfrom(emu::lean_mul(x, k.ls) ^ f);
-        a.x = __dsub_rn(xc, ys);
-        a.y = __dadd_rn(yc, xs);
-        return;
-    }
-    a = flip ? phase_slow<true>(a, q) : phase_slow<false>(a, q);
+    if (!phase_flip_lean(a, flip, k)) a = flip ? phase_slow<true>(a, q) : phase_slow<false>(a, q);
 }
 
 template <int NG>

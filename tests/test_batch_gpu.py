@@ -145,3 +145,37 @@ def test_batch_sampling_on_exact_and_tied_sums(qsl, port, dtype):
     probs, shots = b.run(angles, np.concatenate(us))
     for i in range(ns.size):
         assert np.array_equal(shots[i], want[i]), (i, int(ns[i]))
+
+
+@pytest.mark.parametrize("dtype", [np.complex128, np.complex64])
+@pytest.mark.parametrize("ns,nshots", [([17, 16, 15, 3, 2], 5000), ([18], 1), ([14, 14, 14], 64), ([13, 12, 11, 4], 0)])
+def test_clusters_shots_and_sizes_match_oracle(qsl, port, dtype, ns, nshots):
+    """Batches small enough for several CTAs to share an instance, instances
+    just above, at and below a tile and below a thread's registers, no shots,
+    one, and more than are sorted on the device; equal uniforms, zero and
+    values above the total among them."""
+    rng = np.random.default_rng(len(ns) + nshots)
+    n = np.array(ns, dtype=np.uint32)
+    ls = rng.integers(1, 4, n.size).astype(np.uint32)
+    b = qsl.Batch(n, ls, nshots, dtype=dtype)
+    fp32 = dtype == np.complex64
+    angles = rng.uniform(0, 2 * np.pi, b.angle_count)
+    u = rng.random(n.size * nshots)
+    if nshots > 10:
+        u[::7] = u[3]
+        u[5], u[6] = 0.0, np.nextafter(1.0, 0.0)
+    if fp32:
+        angles = angles.astype(np.float32).astype(np.float64)
+        u = np.minimum(u.astype(np.float32), np.float32(1 - 2.0 ** -24)).astype(np.float64)
+    for shape in [None] + b.shapes()[:2]:
+        if shape:
+            b.set_shape(*shape)
+        probs, shots = b.run(angles, u)
+        at = 0
+        for i, (m, L) in enumerate(zip(n, ls)):
+            cnt = 2 * int(m) * int(L)
+            p, sh = reference_instance(port, int(m), int(L), angles[at:at + cnt], u[i * nshots:(i + 1) * nshots],
+                                       fp32)
+            at += cnt
+            assert np.array_equal(probs[i], p), (shape, i)
+            assert np.array_equal(shots[i], sh), (shape, i)
