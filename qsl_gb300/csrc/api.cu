@@ -138,6 +138,21 @@ int wait_error(qslc_state *s)
     return fail(QSLC_ETIMEOUT, "a staged sweep's shared-memory barrier wait ran out; the state is undefined");
 }
 
+int ensure_pinned(qslc_state *s, size_t bytes)
+{
+    if (s->host_pinned_bytes >= bytes) return QSLC_OK;
+    if (s->host_pinned) cudaFreeHost(s->host_pinned);
+    s->host_pinned = nullptr;
+    s->host_pinned_bytes = 0;
+    if (cudaMallocHost(&s->host_pinned, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        s->host_pinned = nullptr;
+        return fail(QSLC_EOOM, "out of pinned host memory");
+    }
+    s->host_pinned_bytes = bytes;
+    return QSLC_OK;
+}
+
 void Scratch::release()
 {
     if (ptr) cudaFree(ptr);

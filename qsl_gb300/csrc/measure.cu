@@ -17,11 +17,7 @@ template <class T, class A>
 static int prob_t(qslc_state *s, unsigned targ, unsigned outcome, double *out)
 {
     ProdHalf<T> pr{static_cast<const cplx<T> *>(s->amps), targ, uint64_t(outcome) << targ};
-    SeqOut<A> so;
-    int rc = seq_run<ProdHalf<T>, T, A>(s, pr, uint64_t(1) << (s->n - 1), false, so);
-    if (rc) return rc;
-    *out = double(so.total);
-    return QSLC_OK;
+    return seq_total<ProdHalf<T>, T, A>(s, pr, uint64_t(1) << (s->n - 1), out);
 }
 
 int seq_prob(qslc_state *s, unsigned targ, unsigned outcome, double *out)
@@ -35,8 +31,7 @@ template <class T>
 static int sample_all_t(qslc_state *s, const double *u, uint64_t n, uint64_t *out)
 {
     ProdAll<T> pr{static_cast<const cplx<T> *>(s->amps)};
-    auto host_index = [](uint64_t j) { return j; };
-    return seq_sample<ProdAll<T>, T, double>(s, pr, uint64_t(1) << s->n, u, n, out, host_index);
+    return seq_sample<ProdAll<T>, T, double>(s, pr, uint64_t(1) << s->n, u, n, out);
 }
 
 // sampleAll2 (measure.cpp:237-267): an Fp running sum, strict comparison
@@ -44,8 +39,7 @@ template <class T>
 static int sample_all2_t(qslc_state *s, const double *u, uint64_t n, uint64_t *out)
 {
     ProdAll<T> pr{static_cast<const cplx<T> *>(s->amps)};
-    auto host_index = [](uint64_t j) { return j; };
-    return seq_sample<ProdAll<T>, T, T>(s, pr, uint64_t(1) << s->n, u, n, out, host_index, true);
+    return seq_sample<ProdAll<T>, T, T>(s, pr, uint64_t(1) << s->n, u, n, out, true);
 }
 
 int seq_sample_all2(qslc_state *s, const double *u, uint64_t n, uint64_t *out)

@@ -513,11 +513,7 @@ static int np_prob_t(qslc_state *s, unsigned t, unsigned o, double *out)
 {
     NPTables *tb = tables_of(s);
     ProdNPMask<T> pr{static_cast<const cplx<T> *>(s->amps), tb->tab[T_NW], t, o};
-    SeqOut<T> so;
-    int rc = seq_run<ProdNPMask<T>, T, T>(s, pr, s->namps, false, so);
-    if (rc) return rc;
-    *out = double(so.total);
-    return QSLC_OK;
+    return seq_total<ProdNPMask<T>, T, T>(s, pr, s->namps, out);
 }
 
 int np_prob(qslc_state *s, unsigned targ, unsigned outcome, double *out)
@@ -532,10 +528,7 @@ static int np_sample_t(qslc_state *s, const double *u, uint64_t n, uint64_t *out
 {
     NPTables *tb = tables_of(s);
     ProdNPAll<T> pr{static_cast<const cplx<T> *>(s->amps), tb->tab[T_NW]};
-    const unsigned w = s->nones;
-    const unsigned nq = s->n;
-    auto host_index = [nq, w](uint64_t j) -> uint64_t { return unrank_of(j, nq, w); };
-    return seq_sample<ProdNPAll<T>, T, T>(s, pr, s->namps, u, n, out, host_index);
+    return seq_sample<ProdNPAll<T>, T, T>(s, pr, s->namps, u, n, out);
 }
 
 // sampleAll2 over the weight-w sector (np/measure.cpp:259-289)
@@ -544,9 +537,7 @@ static int np_sample2_t(qslc_state *s, const double *u, uint64_t n, uint64_t *ou
 {
     NPTables *tb = tables_of(s);
     ProdNPAll<T> pr{static_cast<const cplx<T> *>(s->amps), tb->tab[T_NW]};
-    const unsigned w = s->nones, nq = s->n;
-    auto host_index = [nq, w](uint64_t j) -> uint64_t { return unrank_of(j, nq, w); };
-    return seq_sample<ProdNPAll<T>, T, T>(s, pr, s->namps, u, n, out, host_index, true);
+    return seq_sample<ProdNPAll<T>, T, T>(s, pr, s->namps, u, n, out, true);
 }
 
 int np_sample_all2(qslc_state *s, const double *u, uint64_t n, uint64_t *out)

@@ -7,25 +7,28 @@
 // the sampling CDF sums every amplitude in ascending order
 // (measure.cpp:60-78).
 //
-// The sum is computed in three device passes over tiles of SEQ_TILE
-// consecutive elements plus a host walk over per-tile metadata:
-//   1. k_seq_tile_sum: an estimate of each tile's sum;
-//   2. the host turns the estimates into a guess of the binade the running
-//      sum occupies in each tile; k_seq_tile_steps counts, per tile, the
-//      grid steps of that binade (replay.cuh) and flags ties;
-//   3. the host walks the tiles in order, advancing the exact running sum by
-//      u_e * D for every tile whose guess holds and replaying the others
-//      term by term (their terms fetched with k_seq_fetch);
-//   4. for sampling, k_seq_resolve rebuilds the exact partial sums inside
-//      each tile that received a shot and finds, for each uniform u, the
-//      first element with partial sum >= u: the reference's binary search
-//      over its Dist vector (measure.cpp:164-188) returns the same element.
+// The sum is computed on the device, in tiles of SEQ_TILE consecutive
+// elements, with one pass over the state and no host step in between:
+//   1. k_seq_estimate: an estimate of each tile's sum from a sample of it;
+//   2. k_seq_guess: from their prefix sums, a guess of the binade the running
+//      sum occupies in each tile;
+//   3. k_seq_steps: the effect of each tile on a running sum of that binade,
+//      in grid steps (replay.cuh) -- which is also the tile's sum to within
+//      rounding;
+//   4. k_seq_guess again, on these sums: the tiles whose guess was wrong go on
+//      a list, and k_seq_steps does them again;
+//   5. k_seq_walk: one CTA walks the tiles in order, a few thousand a round by
+//      a scan of their effects, and advances the exact running sum; the few
+//      tiles in which it crosses a power of two (or whose guess is still
+//      wrong) it walks term by term, in rounds too;
+//   6. for sampling, k_seq_shots: one warp per uniform finds the tile, the
+//      512-term piece and the term whose partial sum is the first to reach
+//      the uniform; the reference's binary search over its Dist vector
+//      (measure.cpp:164-188) returns the same element.
 #pragma once
 
 #include <algorithm>
 #include <cmath>
-#include <unordered_map>
-#include <utility>
 #include <vector>
 
 #include "qslc_internal.cuh"
@@ -36,7 +39,8 @@ namespace qslc {
 constexpr int SEQ_TILE = 4096;
 constexpr int SEQ_TPB = 256;
 constexpr int SEQ_PER = SEQ_TILE / SEQ_TPB;
-constexpr int SEQ_FETCH_CAP = 256;   // tiles fetched per batch for host replay
+constexpr int SEQ_PIECES = SEQ_TPB / 32;   // pieces of a tile: a warp's terms
+constexpr int SEQ_PIECE = SEQ_TILE / SEQ_PIECES;
 
 // ---------------------------------------------------------------------------
 // Producers over the plain 2^n layout.
@@ -66,535 +70,835 @@ struct ProdAll {         // every amplitude, ascending
 };
 
 // ---------------------------------------------------------------------------
-// Kernels.  Element j of tile b is b*SEQ_TILE + k*SEQ_TPB + threadIdx.x for
-// k = 0..SEQ_PER-1, so every load instruction of a warp is coalesced.
+// Scans of transducers.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double warp_sum_d(double v)
 {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ uint64_t warp_sum_u(uint64_t v)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
-template <class Prod>
-__global__ void __launch_bounds__(SEQ_TPB) k_seq_tile_sum(Prod pr, uint64_t count, uint64_t ntiles,
-                                                          double *__restrict__ out)
+__device__ __forceinline__ Tx shfl_up_tx(const Tx &t, unsigned off)
 {
-    __shared__ double red[SEQ_TPB / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint64_t b = blockIdx.x; b < ntiles; b += gridDim.x) {
-        double acc = 0;
-        const uint64_t base = b * SEQ_TILE;
-#pragma unroll 4
-        for (int k = 0; k < SEQ_PER; k++) {
-            uint64_t j = base + uint64_t(k) * SEQ_TPB + threadIdx.x;
-            if (j < count) acc += double(pr.p(j));
-        }
-        acc = warp_sum_d(acc);
-        if (lane == 0) red[warp] = acc;
-        __syncthreads();
-        if (warp == 0) {
-            double v = lane < SEQ_TPB / 32 ? red[lane] : 0.0;
-            v = warp_sum_d(v);
-            if (lane == 0) out[b] = v;
-        }
-        __syncthreads();
-    }
-}
-
-// Packs a term's grid steps with its tie bit (bit 63); steps never reach
-// 2^62 without also raising `big`.
-constexpr uint64_t TIE_BIT = uint64_t(1) << 63;
-
-__device__ __forceinline__ Tx warp_compose(Tx x)
-{
-    // ordered reduction: after the loop lane 0 holds lane 0 then 1 then ... 31
-    const int lane = threadIdx.x & 31;
-    for (int off = 1; off < 32; off <<= 1) {
-        Tx y;
-        y.d[0] = __shfl_down_sync(0xffffffffu, x.d[0], off);
-        y.d[1] = __shfl_down_sync(0xffffffffu, x.d[1], off);
-        if ((lane & (2 * off - 1)) == 0) x = tx_then(x, y);
-    }
-    return x;
+    Tx r;
+    r.d[0] = __shfl_up_sync(0xffffffffu, (unsigned long long)t.d[0], off);
+    r.d[1] = __shfl_up_sync(0xffffffffu, (unsigned long long)t.d[1], off);
+    return r;
 }
 
 __device__ __forceinline__ Tx warp_scan_incl(Tx x)
 {
     // inclusive ordered scan: lane l holds lanes 0..l composed in order
-    const int lane = threadIdx.x & 31;
-    for (int off = 1; off < 32; off <<= 1) {
-        Tx y;
-        y.d[0] = __shfl_up_sync(0xffffffffu, x.d[0], off);
-        y.d[1] = __shfl_up_sync(0xffffffffu, x.d[1], off);
+    const unsigned lane = threadIdx.x & 31;
+    for (unsigned off = 1; off < 32; off <<= 1) {
+        const Tx y = shfl_up_tx(x, off);
         if (lane >= off) x = tx_then(y, x);
     }
     return x;
 }
 
-// Grid steps of every term of a tile into `sm` (coalesced loads), and the
-// OR of the `big` flags.
-template <class Prod, class A>
-__device__ __forceinline__ unsigned tile_terms(const Prod &pr, uint64_t count, uint64_t base, int e,
-                                               uint64_t *sm)
+__device__ __forceinline__ uint64_t warp_min_u(uint64_t v)
 {
-    unsigned big_any = 0;
-#pragma unroll 4
-    for (int k = 0; k < SEQ_PER; k++) {
-        const int i = k * SEQ_TPB + threadIdx.x;
-        const uint64_t j = base + uint64_t(i);
-        uint64_t v = 0;
-        if (j < count) {
-            bool tie, big;
-            v = grid_steps<A>(A(pr.p(j)), e, tie, big);
-            if (big) {
-                big_any = 1;
-                v = 0;
-            }
-            if (tie) v |= TIE_BIT;
-        }
-        sm[i] = v;
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t w = __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
+        v = w < v ? w : v;
     }
-    return big_any;
+    return v;
 }
 
-// The transducer of this thread's SEQ_PER consecutive terms of `sm`.
-__device__ __forceinline__ Tx segment_tx(const uint64_t *sm)
+// ---------------------------------------------------------------------------
+// 1. Estimates.  One warp per tile adds 64 terms, in four pieces spread over
+// the tile: a guess of a binade needs no more, and the pass reads 1/64 of the
+// state.  k_seq_whole adds all of them, one CTA per tile, for the few tiles of
+// a small state.
+// ---------------------------------------------------------------------------
+template <class Prod>
+__global__ void __launch_bounds__(SEQ_TPB) k_seq_estimate(Prod pr, uint64_t count, uint64_t ntiles,
+                                                          double *__restrict__ out)
 {
-    Tx t = tx_identity();
+    const unsigned lane = threadIdx.x & 31;
+    const uint64_t warps = uint64_t(gridDim.x) * (SEQ_TPB / 32);
+    for (uint64_t b = uint64_t(blockIdx.x) * (SEQ_TPB / 32) + (threadIdx.x >> 5); b < ntiles; b += warps) {
+        const uint64_t base = b * SEQ_TILE;
+        double acc = 0, n = 0;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint64_t j = base + (lane >> 3) * (SEQ_TILE / 4) + (lane & 7) + 8 * k;
+            if (j < count) {
+                acc += double(pr.p(j));
+                n += 1;
+            }
+        }
+        acc = warp_sum_d(acc);
+        n = warp_sum_d(n);
+        const double all = double(count - base < uint64_t(SEQ_TILE) ? count - base : uint64_t(SEQ_TILE));
+        if (lane == 0) out[b] = n > 0 ? acc * (all / n) : 0.0;
+    }
+}
+
+template <class Prod>
+__global__ void __launch_bounds__(SEQ_TPB) k_seq_whole(Prod pr, uint64_t count, double *__restrict__ out)
+{
+    __shared__ double red[SEQ_TPB / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t base = uint64_t(blockIdx.x) * SEQ_TILE;
+    double acc = 0;
 #pragma unroll
     for (int k = 0; k < SEQ_PER; k++) {
-        const uint64_t v = sm[threadIdx.x * SEQ_PER + k];
-        t = tx_then(t, tx_term(v & ~TIE_BIT, (v & TIE_BIT) != 0));
+        const uint64_t j = base + uint64_t(k * SEQ_TPB + int(threadIdx.x));
+        if (j < count) acc += double(pr.p(j));
     }
-    return t;
-}
-
-template <class Prod, class A>
-__global__ void __launch_bounds__(SEQ_TPB) k_seq_tile_steps(Prod pr, uint64_t count, uint64_t ntiles,
-                                                            const int16_t *__restrict__ guess,
-                                                            uint64_t *__restrict__ steps,
-                                                            uint8_t *__restrict__ flags)
-{
-    __shared__ uint64_t sm[SEQ_TILE];
-    __shared__ Tx wtx[SEQ_TPB / 32];
-    __shared__ unsigned big_all;
-    constexpr uint64_t CAP = uint64_t(1) << (fp_traits<A>::MANT + 1);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint64_t b = blockIdx.x; b < ntiles; b += gridDim.x) {
-        if (threadIdx.x == 0) big_all = 0;
-        __syncthreads();
-        const unsigned big = tile_terms<Prod, A>(pr, count, b * SEQ_TILE, guess[b], sm);
-        if (big) atomicOr(&big_all, 1u);
-        __syncthreads();
-        Tx t = segment_tx(sm);
-        // a run of 4096 terms below CAP each stays below 2^62: no overflow
-        t = warp_compose(t);
-        if (lane == 0) wtx[warp] = t;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            Tx tot = wtx[0];
-            for (int w = 1; w < SEQ_TPB / 32; w++) tot = tx_then(tot, wtx[w]);
-            unsigned fl = big_all ? 2u : 0u;
-            if (tot.d[0] >= CAP || tot.d[1] >= CAP) fl |= 2u;
-            steps[2 * b] = tot.d[0] < CAP ? tot.d[0] : CAP;
-            steps[2 * b + 1] = tot.d[1] < CAP ? tot.d[1] : CAP;
-            flags[b] = uint8_t(fl);
-        }
-        __syncthreads();
+    acc = warp_sum_d(acc);
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double v = red[0];
+        for (int w = 1; w < SEQ_TPB / 32; w++) v += red[w];
+        out[blockIdx.x] = v;
     }
 }
 
-template <class Prod, class P>
-__global__ void __launch_bounds__(SEQ_TPB) k_seq_fetch(Prod pr, uint64_t count,
-                                                       const uint64_t *__restrict__ tiles, int ntl,
-                                                       P *__restrict__ out)
-{
-    for (int q = blockIdx.x; q < ntl; q += gridDim.x) {
-        const uint64_t base = tiles[q] * SEQ_TILE;
-        for (int i = threadIdx.x; i < SEQ_TILE; i += SEQ_TPB) {
-            uint64_t j = base + i;
-            out[uint64_t(q) * SEQ_TILE + i] = j < count ? pr.p(j) : P(0);
-        }
-    }
-}
+// ---------------------------------------------------------------------------
+// 2, 4. Guesses.  One CTA; thread t takes consecutive tiles.  With `redo`
+// the guesses are compared with the ones the steps were counted for, and the
+// tiles that differ are listed (redo[0]: their number).
+// ---------------------------------------------------------------------------
+constexpr int SEQ_GUESS_TPB = 1024;
 
-struct ResolveItem {
-    uint64_t tile;
-    double start;       // exact running sum before the tile's first element
-    int32_t binade;     // binade the sum stays in throughout the tile
-    uint32_t shot0;     // first shot (index into the sorted uniforms)
-    uint32_t nshot;
-    uint32_t strict;    // 1: first partial sum > u (sampleAll2); 0: >= u (sampleAll)
+enum SeqFlag : uint8_t {
+    SEQ_BIG = 1,       // a term or the tile's steps do not fit the binade
+    SEQ_NONE = 2,      // no guess of a normal binade
+    SEQ_ZERO = 4       // every term is zero
 };
 
-template <class Prod, class A>
-__global__ void __launch_bounds__(SEQ_TPB) k_seq_resolve(Prod pr, uint64_t count,
-                                                         const ResolveItem *__restrict__ items,
-                                                         int nitems,
-                                                         const double *__restrict__ u_sorted,
-                                                         uint64_t *__restrict__ out_sorted)
-{
-    __shared__ uint64_t pre[SEQ_TILE];
-    __shared__ Tx wtx[SEQ_TPB / 32];
-    constexpr int MANT = fp_traits<A>::MANT;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int q = blockIdx.x; q < nitems; q += gridDim.x) {
-        const ResolveItem it = items[q];
-        const uint64_t base = it.tile * SEQ_TILE;
-        tile_terms<Prod, A>(pr, count, base, it.binade, pre);
-        __syncthreads();
-        // running sum before the tile, in grid steps of the tile's binade
-        const uint64_t s0 = uint64_t(ldexp(it.start, MANT - it.binade));
-        const Tx seg = segment_tx(pre);
-        Tx incl = warp_scan_incl(seg);
-        if (lane == 31) wtx[warp] = incl;
-        __syncthreads();
-        Tx before = tx_identity();                 // warps before this one
-        for (int w = 0; w < warp; w++) before = tx_then(before, wtx[w]);
-        Tx excl_in_warp;
-        excl_in_warp.d[0] = __shfl_up_sync(0xffffffffu, incl.d[0], 1);
-        excl_in_warp.d[1] = __shfl_up_sync(0xffffffffu, incl.d[1], 1);
-        if (lane == 0) excl_in_warp = tx_identity();
-        const Tx prefix = tx_then(before, excl_in_warp);
-        const uint64_t off = prefix.d[s0 & 1];
-        uint64_t loc[SEQ_PER];
-        uint64_t run = off;
-#pragma unroll
-        for (int k = 0; k < SEQ_PER; k++) {
-            const uint64_t v = pre[threadIdx.x * SEQ_PER + k];
-            const Tx t = tx_term(v & ~TIE_BIT, (v & TIE_BIT) != 0);
-            run += t.d[(s0 + run) & 1];
-            loc[k] = run;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < SEQ_PER; k++) pre[threadIdx.x * SEQ_PER + k] = loc[k];
-        __syncthreads();
-        for (uint32_t k = threadIdx.x; k < it.nshot; k += SEQ_TPB) {
-            const double u = u_sorted[it.shot0 + k];
-            int lo = 0, hi = SEQ_TILE - 1;   // first i with partial(i) >= u
-            while (lo < hi) {
-                int mid = (lo + hi) >> 1;
-                double v = double(A(ldexp(double(s0 + pre[mid]), it.binade - MANT)));
-                if (it.strict ? (v > u) : (v >= u)) hi = mid;
-                else lo = mid + 1;
-            }
-            const uint64_t last = count - 1 - base;   // the tile's last valid element
-            out_sorted[it.shot0 + k] = pr.index(base + (uint64_t(lo) < last ? uint64_t(lo) : last));
-        }
-        __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Host sequencer.
-// ---------------------------------------------------------------------------
 template <class A>
-struct SeqOut {
-    A total = A(0);
-    std::vector<A> starts;                                  // per tile
-    std::vector<int16_t> guess;
-    std::unordered_map<uint64_t, std::vector<A>> partials;  // replayed tiles
-    uint64_t replayed = 0;
+__global__ void __launch_bounds__(SEQ_GUESS_TPB) k_seq_guess(const double *__restrict__ est, uint64_t ntiles,
+                                                            int16_t *__restrict__ guess, uint32_t *__restrict__ redo,
+                                                            const uint8_t *__restrict__ flags)
+{
+    __shared__ double wsum[32];
+    const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t per = (ntiles + SEQ_GUESS_TPB - 1) / SEQ_GUESS_TPB, b0 = tid * per;
+    const uint64_t b1 = b0 + per < ntiles ? b0 + per : ntiles;
+    double mine = 0;
+    for (uint64_t b = b0; b < b1; b++) mine += est[b];
+    double incl = mine;
+    for (unsigned off = 1; off < 32; off <<= 1) {
+        const double y = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    double run = incl - mine;
+    for (unsigned w = 0; w < warp; w++) run += wsum[w];
+    if (run < 0) run = 0;                              // rounding of incl - mine
+    for (uint64_t b = b0; b < b1; b++) {
+        const double end = run + est[b];
+        const int16_t g = int16_t(binade<A>(A(run > 0 ? run : end)));
+        if (redo) {
+            if (!(flags[b] & SEQ_ZERO) && g != guess[b]) {
+                guess[b] = g;
+                redo[1 + atomicAdd(redo, 1u)] = uint32_t(b);
+            }
+        } else {
+            guess[b] = g;
+        }
+        run = end;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// 3. Steps.  Warp w of a tile's CTA takes the piece of 512 consecutive terms
+// from 512 w on, its lanes 32 consecutive ones at a time, so every load of a
+// warp is coalesced.  Step counts just add up, in any order, unless a term is
+// a rounding tie; a warp with a tie does its piece again, composing the terms
+// in order.
+//
+// Bound by the FP64 pipe (three operations a term, 74% busy) with
+// the integer work on step counts behind it.  Two passes over the state with the sums
+// of the first in FP64, a host step between them and 32-way conflicts in shared
+// memory took 2.3 ms for the probability of one qubit of 28; this and the
+// redone tiles take 1.0.
+// ---------------------------------------------------------------------------
+// Packs a term's grid steps with its tie bit (bit 63); steps never reach
+// 2^62 without also raising `big`.
+constexpr uint64_t TIE_BIT = uint64_t(1) << 63;
+
+// Grid steps of p >= 0 in binade e as grid_steps<A>, packed: the common case
+// (a normal term below the binade, by a shift of less than 64) first.
+template <class A, class P>
+__device__ __forceinline__ uint64_t packed_steps(P p, int e, bool &big)
+{
+    using TP = fp_traits<P>;
+    const auto b = to_bits(p);
+    const int ef = int(b >> TP::MANT);                        // p is not negative
+    const int sh = (e - fp_traits<A>::MANT) - (ef - TP::BIAS - TP::MANT);
+    if (ef > 0 && ef < TP::EXPMASK && sh >= 1 + TP::MANT - fp_traits<A>::MANT && sh >= 1 && sh < 64) {
+        const uint64_t m = uint64_t(b & ((typename TP::bits_t(1) << TP::MANT) - 1)) | (uint64_t(1) << TP::MANT);
+        const uint64_t t = m >> (sh - 1);                     // the steps and the half
+        const bool tie = (t & 1) && (m << (65 - sh)) == 0 && (sh > 1);
+        if (sh == 1) return (t >> 1) | ((t & 1) ? TIE_BIT : 0);
+        return tie ? (t >> 1) | TIE_BIT : (t + 1) >> 1;
+    }
+    bool tie, bg;
+    uint64_t v = grid_steps<A>(p, e, tie, bg);
+    if (bg) {
+        big = true;
+        return 0;
+    }
+    return v | (tie ? TIE_BIT : 0);
+}
+
+// A thread's steps, added up: quick() takes a term by 32-bit shifts of its
+// significand -- twice the steps and a half bit, whose rounding (up, away from
+// a tie) is the half bit again, so a sum of truncated doubles and a count of
+// half bits hold the total -- and declines what needs more: terms of more
+// than half the binade, suspected ties, and every term of a very low binade.
+// 25 instructions a term, with packed_steps alone 60.
+template <class A, class P>
+struct StepSum {
+    uint64_t sum = 0, ties = 0;
+    bool big = false;
+    __device__ __forceinline__ explicit StepSum(int e_) : e(e_) {}
+    __device__ __forceinline__ void add(P p)
+    {
+        const uint64_t v = packed_steps<A>(p, e, big);
+        sum += v & ~TIE_BIT;
+        ties |= v;
+    }
+    __device__ __forceinline__ uint64_t total() const { return sum; }
+    int e;
+};
+template <>
+struct StepSum<double, double> {
+    uint64_t sum = 0, twice = 0, ties = 0;
+    uint32_t odd = 0;
+    bool big = false;
+    __device__ __forceinline__ explicit StepSum(int e_) : e(e_) {}
+    __device__ __forceinline__ void add(double p)
+    {
+        const uint32_t hi = uint32_t(__double2hiint(p)), lo = uint32_t(__double2loint(p));
+        const int k = (e + 1022) - int(hi >> 20);              // bits below the half bit
+        const uint32_t mh = (hi & 0x000FFFFFu) | 0x00100000u;
+        const bool far = k >= 32;
+        const uint32_t tl = far ? __funnelshift_rc(mh, 0u, unsigned(k) - 32u) : __funnelshift_rc(lo, mh, unsigned(k));
+        const uint32_t th = __funnelshift_rc(mh, 0u, unsigned(k));
+        const uint32_t below = far ? lo : lo << (32 - k);
+        // with e + 1022 >= 56 a zero or a subnormal term shifts out whatever
+        // its hidden bit, and with k < 1 (an infinity or NaN too) it declines
+        if (k < 1 || e + 1022 < 56 || ((tl & 1u) && below == 0)) {
+            const uint64_t v = packed_steps<double>(p, e, big);
+            sum += v & ~TIE_BIT;
+            ties |= v;
+        } else {
+            twice += (uint64_t(th) << 32) | tl;
+            odd += tl & 1u;
+        }
+    }
+    __device__ __forceinline__ uint64_t total() const { return sum + ((twice + odd) >> 1); }
+    int e;
 };
 
-// Device working storage for one sequence of `ntiles` tiles, carved from
-// one block; `fetch_cap` tiles of terms can be staged for host replay.
+template <class Prod, class A>
+__global__ void __launch_bounds__(SEQ_TPB, 4) k_seq_steps(Prod pr, uint64_t count, uint64_t ntiles,
+                                                          const int16_t *__restrict__ guess,
+                                                          const uint32_t *__restrict__ redo,
+                                                          uint64_t *__restrict__ steps, uint64_t *__restrict__ pieces,
+                                                          uint8_t *__restrict__ flags, double *__restrict__ est)
+{
+    __shared__ Tx ptx[SEQ_PIECES];
+    __shared__ double psum[SEQ_PIECES];
+    constexpr uint64_t CAP = uint64_t(1) << (fp_traits<A>::MANT + 1);
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t todo = redo ? redo[0] : ntiles;
+    for (uint64_t i = blockIdx.x; i < todo; i += gridDim.x) {
+        const uint64_t b = redo ? redo[1 + i] : i;
+        const uint64_t first = b * SEQ_TILE + warp * SEQ_PIECE + lane;
+        const int e = guess[b];
+        const bool any = e >= fp_traits<A>::EMIN;
+        using P = decltype(pr.p(uint64_t(0)));
+        StepSum<A, P> mine(e);
+        bool nonzero = false;
+#pragma unroll 8
+        for (int k = 0; k < SEQ_PIECE; k += 32) {
+            if (first + k < count) {
+                const P p = pr.p(first + k);
+                nonzero |= to_bits(p) != 0;
+                if (any) mine.add(p);
+            }
+        }
+        bool big = mine.big;
+        uint64_t sum = mine.total();
+        const uint64_t ties = mine.ties;
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, (unsigned long long)sum, o);
+        Tx t{{sum, sum}};
+        if (__any_sync(0xffffffffu, (ties & TIE_BIT) != 0)) {
+            t = tx_identity();
+            for (int k = 0; k < SEQ_PIECE; k += 32) {
+                uint64_t v = 0;
+                if (first + k < count) v = packed_steps<A>(pr.p(first + k), e, big);
+                const Tx inc = warp_scan_incl(tx_term(v & ~TIE_BIT, (v & TIE_BIT) != 0));
+                Tx all;
+                all.d[0] = __shfl_sync(0xffffffffu, (unsigned long long)inc.d[0], 31);
+                all.d[1] = __shfl_sync(0xffffffffu, (unsigned long long)inc.d[1], 31);
+                t = tx_then(t, all);
+            }
+        }
+        if (lane == 0) {
+            ptx[warp] = t;
+            if (pieces) {
+                pieces[2 * (b * SEQ_PIECES + warp)] = t.d[0];
+                pieces[2 * (b * SEQ_PIECES + warp) + 1] = t.d[1];
+            }
+        }
+        const bool big_all = __syncthreads_or(big) != 0;
+        const bool some = __syncthreads_or(nonzero) != 0;
+        const bool lost = big_all || (!any && some);
+        if (lost) {                                       // the steps do not give the tile's sum
+            double acc = 0;
+            for (int k = 0; k < SEQ_PIECE; k += 32)
+                if (first + k < count) acc += double(pr.p(first + k));
+            acc = warp_sum_d(acc);
+            if (lane == 0) psum[warp] = acc;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            Tx tot = ptx[0];
+            for (int w = 1; w < SEQ_PIECES; w++) tot = tx_then(tot, ptx[w]);
+            uint8_t fl = 0;
+            if (!some) fl = SEQ_ZERO;
+            else if (!any) fl = SEQ_NONE;
+            else if (big_all || tot.d[0] >= CAP || tot.d[1] >= CAP) fl = SEQ_BIG;
+            steps[2 * b] = tot.d[0];
+            steps[2 * b + 1] = tot.d[1];
+            flags[b] = fl;
+            double sum_est = 0;
+            if (lost)
+                for (int w = 0; w < SEQ_PIECES; w++) sum_est += psum[w];
+            else if (some) sum_est = ldexp(double(tot.d[0]), e - fp_traits<A>::MANT);
+            est[b] = sum_est;
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// 5. The walk.
+// ---------------------------------------------------------------------------
+// Threads: fewer leave the SM idle in the terms, more wait longer in the scans
+// (ten probabilities of a 28-qubit state walk in 4.5 / 3.4 / 3.1 / 3.7 ms with
+// 128 / 256 / 512 / 1024).
+constexpr int SEQ_WALK_TPB = 512, SEQ_WALK_WARPS = SEQ_WALK_TPB / 32;
+constexpr int SEQ_RUN = 16;                            // tiles a thread takes per round
+constexpr int SEQ_TERMS = SEQ_TILE / SEQ_WALK_TPB;     // most terms a thread takes of a tile per round
+constexpr uint64_t SEQ_END = ~uint64_t(0);
+
+template <class A> __device__ __forceinline__ A from_bits(uint64_t b);
+template <> __device__ __forceinline__ double from_bits<double>(uint64_t b) { return __longlong_as_double((long long)b); }
+template <> __device__ __forceinline__ float from_bits<float>(uint64_t b) { return __uint_as_float(uint32_t(b)); }
+
+template <class A> struct rn_add;
+template <> struct rn_add<double> {
+    static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+};
+template <> struct rn_add<float> {
+    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+};
+
+// Grid positions from this one up lie outside any binade; counts are capped
+// here, so that the sums of a scan over the CTA stay below 2^62.
+constexpr uint64_t SEQ_CAP = uint64_t(1) << 54;
+
+struct WalkShared {
+    uint64_t count[2][SEQ_WALK_WARPS];
+    Tx tx[SEQ_WALK_WARPS];
+    uint64_t least[SEQ_WALK_WARPS];
+    uint64_t pos, at;        // where a round ended: the position (or sum) and the next item
+};
+
+__device__ __forceinline__ uint64_t block_min(uint64_t v, WalkShared &sh)
+{
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = warp_min_u(v);
+    __syncthreads();
+    if (lane == 0) sh.least[warp] = v;
+    __syncthreads();
+    return warp_min_u(sh.least[lane % SEQ_WALK_WARPS]);
+}
+
+// The effect on a sum of what the threads before this one add: this thread's
+// steps when the sum is even or odd (they differ only with a rounding tie).
+// Returns the grid position before this thread's part, given the round's
+// start m0.  One barrier when no thread has a tie; `turn` alternates.
+__device__ __forceinline__ uint64_t scan_from(uint64_t m0, Tx mine, WalkShared &sh, unsigned turn)
+{
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t incl = mine.d[0] < SEQ_CAP ? mine.d[0] : SEQ_CAP;
+    const uint64_t own = incl;
+    for (unsigned off = 1; off < 32; off <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, (unsigned long long)incl, off);
+        if (lane >= off) incl += y;
+    }
+    if (lane == 31) sh.count[turn][warp] = incl < SEQ_CAP ? incl : SEQ_CAP;
+    if (!__syncthreads_or(mine.d[0] != mine.d[1])) {
+        uint64_t before = 0;
+#pragma unroll
+        for (unsigned w = 0; w < SEQ_WALK_WARPS; w++)
+            if (w < warp) before += sh.count[turn][w];
+        return m0 + before + (incl - own);
+    }
+    const Tx inc = warp_scan_incl(mine);
+    if (lane == 31) sh.tx[warp] = inc;
+    __syncthreads();
+    Tx before = tx_identity(), excl = shfl_up_tx(inc, 1);
+    for (unsigned w = 0; w < warp; w++) before = tx_then(before, sh.tx[w]);
+    __syncthreads();                                   // sh.tx is read
+    if (lane == 0) excl = tx_identity();
+    excl = tx_then(before, excl);
+    return m0 + excl.d[m0 & 1];
+}
+
+template <class A>
+__device__ __forceinline__ bool finite_sum(A s)
+{
+    return int((to_bits(s) >> fp_traits<A>::MANT) & fp_traits<A>::EXPMASK) != fp_traits<A>::EXPMASK;
+}
+
+// The exact running sum after the terms tm[0..valid) from `s`; every thread
+// returns it.  A sum that starts at zero leaves a binade every time the number
+// of terms doubles: its rounds span four times the terms before them.
+// Where term i lies in shared memory: a gap after every 16, so that threads
+// with 16 (or 8) consecutive terms each read from different banks.
+__device__ __forceinline__ unsigned term_slot(unsigned i) { return i + (i >> 4); }
+
+template <class A, class P>
+__device__ A walk_terms(const P *tm, unsigned valid, A s, WalkShared &sh, unsigned &turn)
+{
+    constexpr uint64_t LIM = uint64_t(1) << (fp_traits<A>::MANT + 1);
+    const unsigned tid = threadIdx.x;
+    const bool small = s == A(0);
+    unsigned i = 0, per = small ? 1 : SEQ_TERMS;
+    while (i < valid) {
+        const int e = binade(s);
+        if (!finite_sum(s)) {
+            // an infinity or a NaN only changes at a NaN
+            bool nan = false;
+            for (unsigned r = i + tid; r < valid; r += SEQ_WALK_TPB) nan |= tm[term_slot(r)] != tm[term_slot(r)];
+            if (__syncthreads_or(nan)) s = A(s + A(NAN));
+            return s;
+        }
+        if (e < fp_traits<A>::EMIN) {
+            if (s == A(0)) {
+                // skip to the first nonzero term
+                uint64_t nz = SEQ_END;
+                for (unsigned r = i + tid; r < valid && nz == SEQ_END; r += SEQ_WALK_TPB)
+                    if (to_bits(tm[term_slot(r)]) != 0) nz = r;
+                nz = block_min(nz, sh);
+                if (nz == SEQ_END) return s;
+                i = unsigned(nz);
+            }
+            s = rn_add<A>::add(s, A(tm[term_slot(i)]));       // zero or subnormal: one term
+            i++;
+            continue;
+        }
+        // a round of terms [i, end) in binade e; the thread in whose terms the
+        // sum leaves the binade walks them and adds the one that does
+        const unsigned most = i + SEQ_WALK_TPB * per, end = most < valid ? most : valid;
+        const unsigned lo = i + tid * per, hi = lo + per < end ? lo + per : end;
+        StepSum<A, P> steps(e);
+        for (unsigned r = lo; r < hi; r++) steps.add(tm[term_slot(r)]);
+        const uint64_t ties = steps.ties;
+        Tx mine;
+        mine.d[0] = steps.big ? SEQ_CAP : steps.total();     // one term leaves the binade by itself
+        mine.d[1] = mine.d[0];
+        auto term = [&](unsigned r) {
+            bool big = false;
+            const uint64_t v = packed_steps<A>(tm[term_slot(r)], e, big);
+            return big ? Tx{{SEQ_CAP, SEQ_CAP}} : tx_term(v & ~TIE_BIT, (v & TIE_BIT) != 0);
+        };
+        if (ties & TIE_BIT) {
+            mine = tx_identity();
+            for (unsigned r = lo; r < hi; r++) mine = tx_then(mine, term(r));
+        }
+        uint64_t pos = scan_from(grid_pos(s), mine, sh, turn);
+        turn ^= 1;
+        if (lo < hi && pos < LIM) {
+            if (pos + mine.d[pos & 1] >= LIM) {    // the one thread where it crosses
+                unsigned r = lo;
+                for (; r + 1 < hi; r++) {
+                    const uint64_t step = term(r).d[pos & 1];
+                    if (pos + step >= LIM) break;
+                    pos += step;
+                }
+                sh.pos = to_bits(rn_add<A>::add(grid_at<A>(pos, e), A(tm[term_slot(r)])));
+                sh.at = r + 1;
+            } else if (hi == end) {
+                sh.pos = to_bits(grid_at<A>(pos + mine.d[pos & 1], e));
+                sh.at = end;
+            }
+        }
+        __syncthreads();
+        s = from_bits<A>(sh.pos);
+        i = unsigned(sh.at);
+        if (small) per = i < 64 ? 1 : i >= 64 * SEQ_TERMS ? SEQ_TERMS : (i + 63) / 64;
+    }
+    return s;
+}
+
+// starts (or null): the running sum before each tile; inside[b]: the binade
+// it stays in throughout tile b, or EMIN - 1 where the tile was walked term
+// by term.  out: the total.
+template <class Prod, class P, class A>
+__global__ void __launch_bounds__(SEQ_WALK_TPB) k_seq_walk(Prod pr, uint64_t count, uint64_t ntiles,
+                                                           const int16_t *__restrict__ guess,
+                                                           const uint64_t *__restrict__ steps,
+                                                           const uint8_t *__restrict__ flags,
+                                                           double *__restrict__ starts, int16_t *__restrict__ inside,
+                                                           double *__restrict__ out)
+{
+    __shared__ P tm[SEQ_TILE + SEQ_TILE / 16];
+    __shared__ WalkShared sh;
+    constexpr uint64_t LIM = uint64_t(1) << (fp_traits<A>::MANT + 1);
+    const unsigned tid = threadIdx.x;
+    A s = A(0);
+    uint64_t t = 0;
+    unsigned turn = 0;
+    while (t < ntiles) {
+        const int e = binade(s);
+        uint64_t bad = t;
+        if (s == A(0)) {
+            // to the first tile that is not all zeros
+            const uint64_t most = t + uint64_t(SEQ_WALK_TPB) * SEQ_RUN;
+            const uint64_t end = most < ntiles ? most : ntiles;
+            uint64_t some = SEQ_END;
+            for (uint64_t b = t + tid; b < end; b += SEQ_WALK_TPB)
+                if (some == SEQ_END && !(flags[b] & SEQ_ZERO)) some = b;
+            some = block_min(some, sh);
+            const uint64_t stop = some == SEQ_END ? end : some;
+            if (starts)
+                for (uint64_t b = t + tid; b < stop; b += SEQ_WALK_TPB) {
+                    starts[b] = 0.0;
+                    inside[b] = int16_t(fp_traits<A>::EMIN - 1);
+                }
+            t = stop;
+            bad = some;
+        } else if (e >= fp_traits<A>::EMIN && finite_sum(s)) {
+            // a round of tiles [t, end) that stay in binade e
+            const uint64_t most = t + uint64_t(SEQ_WALK_TPB) * SEQ_RUN;
+            const uint64_t end = most < ntiles ? most : ntiles;
+            const int per = int((end - t + SEQ_WALK_TPB - 1) / SEQ_WALK_TPB);
+            const uint64_t b0 = t + uint64_t(tid) * unsigned(per);
+            auto effect = [&](uint64_t b) {
+                const uint8_t f = flags[b];
+                const int g = guess[b];
+                const ulonglong2 d = reinterpret_cast<const ulonglong2 *>(steps)[b];
+                if (f & SEQ_ZERO) return tx_identity();
+                if (f || g != e) return Tx{{LIM, LIM}};      // stops here
+                return Tx{{d.x < LIM ? d.x : LIM, d.y < LIM ? d.y : LIM}};
+            };
+            Tx mine = tx_identity();
+            bool parity = false;
+#pragma unroll 4
+            for (int r = 0; r < per; r++)
+                if (b0 + r < end) {
+                    const Tx x = effect(b0 + r);
+                    parity |= x.d[0] != x.d[1];
+                    mine.d[0] += x.d[0];
+                }
+            mine.d[1] = mine.d[0];
+            if (parity) {
+                mine = tx_identity();
+                for (int r = 0; r < per; r++)
+                    if (b0 + r < end) mine = tx_then(mine, effect(b0 + r));
+            }
+            uint64_t pos = scan_from(grid_pos(s), mine, sh, turn);
+            turn ^= 1;
+            if (b0 < end && pos < LIM) {
+                const uint64_t last = b0 + unsigned(per) < end ? b0 + unsigned(per) : end;
+                const uint64_t fin = pos + mine.d[pos & 1];
+                if (fin >= LIM || starts) {                  // the tile the round stops before; the starts
+                    uint64_t b = b0;
+                    for (; b < last; b++) {
+                        const uint64_t d = effect(b).d[pos & 1];
+                        if (pos + d >= LIM) break;
+                        if (starts) {
+                            starts[b] = double(grid_at<A>(pos, e));
+                            inside[b] = int16_t(e);
+                        }
+                        pos += d;
+                    }
+                    if (b < last || last == end) {
+                        sh.pos = pos;
+                        sh.at = b;
+                    }
+                } else if (last == end) {
+                    sh.pos = fin;
+                    sh.at = end;
+                }
+            }
+            __syncthreads();
+            s = grid_at<A>(sh.pos, e);
+            t = sh.at;
+            bad = t < end ? t : SEQ_END;
+        }
+        if (bad == SEQ_END) continue;
+        // tile t term by term
+        if (starts && tid == 0) {
+            starts[t] = double(s);
+            inside[t] = int16_t(fp_traits<A>::EMIN - 1);
+        }
+        if (!(flags[t] & SEQ_ZERO)) {
+            const uint64_t base = t * SEQ_TILE;
+            const unsigned valid = unsigned(count - base < uint64_t(SEQ_TILE) ? count - base : uint64_t(SEQ_TILE));
+            __syncthreads();
+            P v[SEQ_TERMS];
+#pragma unroll
+            for (int r = 0; r < SEQ_TERMS; r++) {
+                const unsigned i = unsigned(r) * SEQ_WALK_TPB + tid;
+                v[r] = i < valid ? pr.p(base + i) : P(0);
+            }
+#pragma unroll
+            for (int r = 0; r < SEQ_TERMS; r++) tm[term_slot(unsigned(r) * SEQ_WALK_TPB + tid)] = v[r];
+            __syncthreads();
+            s = walk_terms<A, P>(tm, valid, s, sh, turn);
+            __syncthreads();
+        }
+        t++;
+    }
+    if (tid == 0) *out = double(s);
+}
+
+// ---------------------------------------------------------------------------
+// 6. Shots: one warp per uniform.
+// ---------------------------------------------------------------------------
+template <class Prod, class A>
+__global__ void __launch_bounds__(SEQ_TPB) k_seq_shots(Prod pr, uint64_t count, uint64_t ntiles,
+                                                       const double *__restrict__ starts,
+                                                       const int16_t *__restrict__ inside,
+                                                       const uint64_t *__restrict__ pieces,
+                                                       const double *__restrict__ total, const double *__restrict__ u,
+                                                       uint32_t nshots, int strict, uint64_t *__restrict__ out)
+{
+    const uint32_t shot = blockIdx.x * (SEQ_TPB / 32) + (threadIdx.x >> 5);
+    const unsigned lane = threadIdx.x & 31;
+    if (shot >= nshots) return;
+    const double x = u[shot];
+    auto reaches = [strict, x](double v) { return strict ? v > x : v >= x; };
+    if (!reaches(*total)) {                                // past the total (:167, :258)
+        if (lane == 0) out[shot] = strict ? ~uint64_t(0) : 0;
+        return;
+    }
+    if (reaches(0.0)) {                                    // the first partial sum does
+        if (lane == 0) out[shot] = pr.index(0);
+        return;
+    }
+    // the first tile whose end reaches x
+    uint64_t lo = 0, hi = ntiles - 1;
+    while (lo < hi) {
+        const uint64_t mid = (lo + hi) >> 1;
+        if (reaches(starts[mid + 1])) hi = mid;
+        else lo = mid + 1;
+    }
+    const uint64_t b = lo;
+    A s = A(starts[b]);
+    uint64_t i = b * SEQ_TILE;
+    const uint64_t tile_end = i + SEQ_TILE < count ? i + SEQ_TILE : count;
+    // first grid position of binade e whose value reaches x
+    auto target = [strict, x](int e) {
+        const A xa = A(x);
+        uint64_t g;
+        if (sizeof(A) == 8 || double(xa) == x) g = grid_ceil<A>(xa, e);
+        else g = grid_ceil<A>(double(xa) < x ? A(__uint_as_float(__float_as_uint(float(xa)) + 1u)) : xa, e);
+        if (strict && ldexp(double(g), e - fp_traits<A>::MANT) == x) g++;
+        return g;
+    };
+    const int e0 = inside[b];
+    if (e0 >= fp_traits<A>::EMIN) {
+        // to the piece that reaches it
+        const uint64_t tgt = target(e0);
+        uint64_t pos = grid_pos(s);
+        for (int w = 0; w + 1 < SEQ_PIECES; w++) {
+            const ulonglong2 d = reinterpret_cast<const ulonglong2 *>(pieces)[b * SEQ_PIECES + w];
+            const uint64_t next = pos + ((pos & 1) ? d.y : d.x);
+            if (next >= tgt) break;
+            pos = next;
+            i += SEQ_PIECE;
+        }
+        s = grid_at<A>(pos, e0);
+    }
+    // the terms from i on, a round of 32 x SEQ_PER at a time
+    uint64_t found = tile_end - 1;
+    while (i < tile_end) {
+        const int e = binade(s);
+        if (e < fp_traits<A>::EMIN || !finite_sum(s)) {
+            if (s == A(0)) {
+                // past zero terms, 32 at a time (a zero sum reaches no x > 0)
+                const uint64_t j = i + lane;
+                const unsigned nz = __ballot_sync(0xffffffffu, j < tile_end && to_bits(pr.p(j)) != 0);
+                if (!nz) {
+                    i += 32;
+                    continue;
+                }
+                i += unsigned(__ffs(nz) - 1);
+            }
+            s = rn_add<A>::add(s, A(pr.p(i)));
+            if (reaches(double(s))) {
+                found = i;
+                break;
+            }
+            i++;
+            continue;
+        }
+        const uint64_t end = i + 32 * SEQ_PER < tile_end ? i + 32 * SEQ_PER : tile_end;
+        const uint64_t base = i + uint64_t(lane) * SEQ_PER;
+        const unsigned len = base < end ? unsigned(end - base < uint64_t(SEQ_PER) ? end - base : SEQ_PER) : 0u;
+        auto run = [&pr, base](unsigned r) { return pr.p(base + r); };
+        bool big = false;
+        const Tx incl = warp_scan_incl(run_effect<A>(run, len, e, big));
+        Tx excl = shfl_up_tx(incl, 1);
+        if (lane == 0) excl = tx_identity();
+        const uint64_t m0 = grid_pos(s);
+        const uint64_t pos0 = m0 + excl.d[m0 & 1];
+        uint64_t pos = pos0;
+        const unsigned walked = run_walk<A>(run, len, e, pos);
+        const uint64_t bad = warp_min_u(walked < len ? base + walked : SEQ_END);
+        const uint64_t stop = bad == SEQ_END ? end : bad;
+        const uint64_t tgt = target(e);
+        const unsigned hit = __ballot_sync(0xffffffffu, len && base < stop && pos >= tgt);
+        if (hit) {
+            const unsigned L = unsigned(__ffs(hit) - 1);
+            uint64_t j = 0;
+            if (lane == L) j = base + run_find<A>(run, len, e, pos0, tgt);
+            found = __shfl_sync(0xffffffffu, (unsigned long long)j, L);
+            break;
+        }
+        const uint64_t last = bad == SEQ_END ? end - 1 : stop;
+        const uint64_t pend = __shfl_sync(0xffffffffu, (unsigned long long)pos, unsigned((last - i) / SEQ_PER));
+        s = grid_at<A>(pend, e);
+        i = stop;
+        if (bad != SEQ_END) {
+            s = rn_add<A>::add(s, A(pr.p(i)));             // the term that leaves the binade
+            if (reaches(double(s))) {
+                found = i;
+                break;
+            }
+            i++;
+        }
+    }
+    if (lane == 0) out[shot] = pr.index(found);
+}
+
+// ---------------------------------------------------------------------------
+// Host side: working storage carved from one block, and the launches.
+// ---------------------------------------------------------------------------
 struct SeqScratch {
-    double *tile_sum;
+    double *total;          // 8 bytes
+    double *est;
+    uint64_t *steps;        // two per tile
     int16_t *guess;
-    uint64_t *steps;
     uint8_t *flags;
-    uint64_t *fetch_ids;
-    void *fetch_buf;
+    uint32_t *redo;         // a count, then up to one entry per tile
+    double *starts;         // sampling only, from here on
+    int16_t *inside;
+    uint64_t *pieces;
     size_t bytes;
     static size_t align(size_t x) { return (x + 255) & ~size_t(255); }
-    static SeqScratch carve(void *base, uint64_t ntiles, size_t p_bytes, int fetch_cap)
+    static SeqScratch carve(void *base, uint64_t ntiles, bool sampling)
     {
         SeqScratch s{};
         char *p = static_cast<char *>(base);
         size_t off = 0;
-        s.tile_sum = reinterpret_cast<double *>(p + off); off += align(ntiles * 8);
-        s.steps = reinterpret_cast<uint64_t *>(p + off); off += align(ntiles * 16);
-        s.guess = reinterpret_cast<int16_t *>(p + off); off += align(ntiles * 2);
-        s.flags = reinterpret_cast<uint8_t *>(p + off); off += align(ntiles);
-        s.fetch_ids = reinterpret_cast<uint64_t *>(p + off); off += align(size_t(fetch_cap) * 8);
-        s.fetch_buf = p + off; off += align(size_t(fetch_cap) * SEQ_TILE * p_bytes);
+        auto take = [&](auto *&q, size_t n) {
+            q = reinterpret_cast<std::remove_reference_t<decltype(q)>>(p + off);
+            off += align(n);
+        };
+        take(s.total, 8);
+        take(s.est, ntiles * 8);
+        take(s.steps, ntiles * 16);
+        take(s.guess, ntiles * 2);
+        take(s.flags, ntiles);
+        take(s.redo, (ntiles + 1) * 4);
+        if (sampling) {
+            take(s.starts, ntiles * 8);
+            take(s.inside, ntiles * 2);
+            take(s.pieces, ntiles * SEQ_PIECES * 16);
+        }
         s.bytes = off;
         return s;
     }
 };
 
-// Host working storage of the walk: per-tile metadata and a small cache of
-// staged tiles (`cap` slots of SEQ_TILE terms each).
-template <class P>
-struct SeqHost {
-    double *est;
-    uint64_t *steps;
-    uint8_t *flags;
-    int16_t *guess;
-    uint8_t *predicted;
-    uint64_t *slot_tile;    // cap entries
-    uint64_t *batch;        // cap entries
-    P *slot_terms;          // cap * SEQ_TILE
-    int cap;
-};
-
-// Where a sequence runs: stream, launch counter, device and host storage.
-template <class P>
-struct SeqEnv {
-    cudaStream_t stream;
-    uint64_t *launches;
-    SeqScratch dev;
-    SeqHost<P> host;
-    int fetch_cap;
-};
-
-template <class A>
-inline A grid_value(uint64_t steps, int e)
+// The sum of producer `pr` over `count` elements, left in sc.total.
+template <class Prod, class P, class A>
+int seq_launch(cudaStream_t str, uint64_t *launches, const SeqScratch &sc, const Prod &pr, uint64_t count)
 {
-    return A(std::ldexp(double(steps), e - fp_traits<A>::MANT));
-}
-
-// The exact sequential sum of producer `pr` over `count` elements.
-// starts (optional, ntiles entries): the running sum before each tile.
-// on_replay (optional): called with (tile, partial sums) for replayed tiles.
-template <class Prod, class P, class A, class OnReplay>
-int seq_core(SeqEnv<P> &env, const Prod &pr, uint64_t count, A *total, A *starts,
-             OnReplay on_replay, uint64_t *replayed)
-{
-    using T = fp_traits<A>;
     const uint64_t ntiles = (count + SEQ_TILE - 1) / SEQ_TILE;
-    SeqScratch &sc = env.dev;
-    SeqHost<P> &h = env.host;
-    cudaStream_t str = env.stream;
-    const unsigned grid = unsigned(std::min<uint64_t>(ntiles, uint64_t(sm_count()) * 8));
-
-    // pass 1: estimates of the tile sums
-    k_seq_tile_sum<Prod><<<grid, SEQ_TPB, 0, str>>>(pr, count, ntiles, sc.tile_sum);
-    (*env.launches)++;
-    QSLC_CUDA(cudaGetLastError());
-    QSLC_CUDA(cudaMemcpyAsync(h.est, sc.tile_sum, ntiles * 8, cudaMemcpyDeviceToHost, str));
-    QSLC_CUDA(cudaStreamSynchronize(str));
-
-    // guesses: the binade of the estimated running sum at each tile start
-    {
-        double run = 0;
-        for (uint64_t b = 0; b < ntiles; b++) {
-            const double end = run + h.est[b];
-            h.guess[b] = int16_t(T::EMIN - 1);
-            h.predicted[b] = 0;
-            if (h.est[b] != 0) {
-                int g0 = binade<A>(A(run)), g1 = binade<A>(A(end));
-                h.guess[b] = int16_t(run > 0 ? g0 : g1);
-                // near or across a power of two: expect a replay
-                double nxt = std::ldexp(1.0, (run > 0 ? g0 : g1) + 1);
-                double margin = (sizeof(A) == 8 ? 1e-9 : 1e-4) * nxt;
-                if (run <= 0 || g0 != g1 || end + margin >= nxt || g0 < T::EMIN) h.predicted[b] = 1;
-            }
-            run = end;
-        }
+    // few tiles: their sums are read whole, and need no second look
+    const bool whole = ntiles <= 512;
+    const unsigned wgrid = unsigned(std::min<uint64_t>((ntiles + SEQ_TPB / 32 - 1) / (SEQ_TPB / 32), sm_count() * 8));
+    const unsigned grid = unsigned(std::min<uint64_t>(ntiles, uint64_t(sm_count()) * 6));
+    if (whole) k_seq_whole<Prod><<<unsigned(ntiles), SEQ_TPB, 0, str>>>(pr, count, sc.est);
+    else k_seq_estimate<Prod><<<wgrid, SEQ_TPB, 0, str>>>(pr, count, ntiles, sc.est);
+    k_seq_guess<A><<<1, SEQ_GUESS_TPB, 0, str>>>(sc.est, ntiles, sc.guess, nullptr, nullptr);
+    k_seq_steps<Prod, A><<<grid, SEQ_TPB, 0, str>>>(pr, count, ntiles, sc.guess, nullptr, sc.steps, sc.pieces, sc.flags,
+                                                    sc.est);
+    *launches += 4;
+    if (!whole) {
+        QSLC_CUDA(cudaMemsetAsync(sc.redo, 0, 4, str));
+        k_seq_guess<A><<<1, SEQ_GUESS_TPB, 0, str>>>(sc.est, ntiles, sc.guess, sc.redo, sc.flags);
+        k_seq_steps<Prod, A><<<grid, SEQ_TPB, 0, str>>>(pr, count, ntiles, sc.guess, sc.redo, sc.steps, sc.pieces,
+                                                        sc.flags, sc.est);
+        *launches += 2;
     }
-    QSLC_CUDA(cudaMemcpyAsync(sc.guess, h.guess, ntiles * 2, cudaMemcpyHostToDevice, str));
-    k_seq_tile_steps<Prod, A><<<grid, SEQ_TPB, 0, str>>>(pr, count, ntiles, sc.guess, sc.steps, sc.flags);
-    (*env.launches)++;
+    k_seq_walk<Prod, P, A><<<1, SEQ_WALK_TPB, 0, str>>>(pr, count, ntiles, sc.guess, sc.steps, sc.flags, sc.starts,
+                                                        sc.inside, sc.total);
     QSLC_CUDA(cudaGetLastError());
-    QSLC_CUDA(cudaMemcpyAsync(h.steps, sc.steps, ntiles * 16, cudaMemcpyDeviceToHost, str));
-    QSLC_CUDA(cudaMemcpyAsync(h.flags, sc.flags, ntiles, cudaMemcpyDeviceToHost, str));
-    QSLC_CUDA(cudaStreamSynchronize(str));
-
-    // Staged terms for replays: a tile that needs one is fetched together
-    // with the next tiles expected to need one, up to `cap` per batch.
-    for (int i = 0; i < h.cap; i++) h.slot_tile[i] = ~uint64_t(0);
-    auto terms_of = [&](uint64_t b, const P **out) -> int {
-        for (int i = 0; i < h.cap; i++)
-            if (h.slot_tile[i] == b) {
-                *out = h.slot_terms + size_t(i) * SEQ_TILE;
-                return QSLC_OK;
-            }
-        int cnt = 0;
-        h.batch[cnt++] = b;
-        for (uint64_t c = b + 1; c < ntiles && cnt < h.cap; c++)
-            if (h.est[c] != 0 && (h.predicted[c] || h.flags[c])) h.batch[cnt++] = c;
-        QSLC_CUDA(cudaMemcpyAsync(sc.fetch_ids, h.batch, size_t(cnt) * 8, cudaMemcpyHostToDevice, str));
-        k_seq_fetch<Prod, P><<<unsigned(std::min(cnt, 1024)), SEQ_TPB, 0, str>>>(
-            pr, count, sc.fetch_ids, cnt, static_cast<P *>(sc.fetch_buf));
-        (*env.launches)++;
-        QSLC_CUDA(cudaGetLastError());
-        QSLC_CUDA(cudaMemcpyAsync(h.slot_terms, sc.fetch_buf, size_t(cnt) * SEQ_TILE * sizeof(P),
-                                  cudaMemcpyDeviceToHost, str));
-        QSLC_CUDA(cudaStreamSynchronize(str));
-        for (int i = 0; i < h.cap; i++) h.slot_tile[i] = i < cnt ? h.batch[i] : ~uint64_t(0);
-        *out = h.slot_terms;
-        return QSLC_OK;
-    };
-
-    // the walk
-    A sum = A(0);
-    uint64_t nrep = 0;
-    const uint64_t cap = uint64_t(1) << (T::MANT + 1);
-    for (uint64_t b = 0; b < ntiles; b++) {
-        if (starts) starts[b] = sum;
-        if (h.est[b] == 0) continue;            // every term is zero
-        const int e = h.guess[b];
-        bool ok = h.flags[b] == 0 && sum > A(0) && binade<A>(sum) == e && e >= T::EMIN;
-        if (ok) {
-            const uint64_t s0 = uint64_t(std::ldexp(double(sum), T::MANT - e));
-            const uint64_t d = h.steps[2 * b + (s0 & 1)];   // ties round to even
-            ok = s0 + d < cap;
-            if (ok) {
-                sum = grid_value<A>(s0 + d, e);
-                continue;
-            }
-        }
-        // replay term by term, exactly as the reference adds them
-        const P *t = nullptr;
-        int r = terms_of(b, &t);
-        if (r) return r;
-        const uint64_t valid = std::min<uint64_t>(SEQ_TILE, count - b * SEQ_TILE);
-        const A before = sum;
-        for (uint64_t i = 0; i < valid; i++) {
-            volatile A next = sum + A(t[i]);
-            sum = next;
-        }
-        on_replay(b, before, t, valid);
-        nrep++;
-    }
-    *total = sum;
-    if (replayed) *replayed = nrep;
     return QSLC_OK;
 }
 
-// The same over a handle's growable scratch; the host storage is heap.
+// The sum over a handle's growable scratch, on the host.
 template <class Prod, class P, class A>
-int seq_run(qslc_state *s, const Prod &pr, uint64_t count, bool keep_partials, SeqOut<A> &out)
+int seq_total(qslc_state *s, const Prod &pr, uint64_t count, double *out)
 {
     const uint64_t ntiles = (count + SEQ_TILE - 1) / SEQ_TILE;
-    const int cap = SEQ_FETCH_CAP;
-    SeqScratch probe = SeqScratch::carve(nullptr, ntiles, sizeof(P), cap);
-    int rc = s->scratch.ensure(probe.bytes);
+    int rc = s->scratch.ensure(SeqScratch::carve(nullptr, ntiles, false).bytes);
+    if (!rc) rc = ensure_pinned(s, 8);
     if (rc) return rc;
-    std::vector<double> est(ntiles);
-    std::vector<uint64_t> steps(2 * ntiles), slot_tile(cap), batch(cap);
-    std::vector<uint8_t> flags(ntiles), predicted(ntiles);
-    out.guess.assign(ntiles, 0);
-    std::vector<P> slot_terms(size_t(cap) * SEQ_TILE);
-    SeqEnv<P> env{s->stream, &s->launches, SeqScratch::carve(s->scratch.ptr, ntiles, sizeof(P), cap),
-                  SeqHost<P>{est.data(), steps.data(), flags.data(), out.guess.data(), predicted.data(),
-                             slot_tile.data(), batch.data(), slot_terms.data(), cap},
-                  cap};
-    out.starts.assign(ntiles, A(0));
-    out.partials.clear();
-    auto on_replay = [&](uint64_t b, A before, const P *t, uint64_t valid) {
-        if (!keep_partials) return;
-        std::vector<A> part(SEQ_TILE);
-        A run = before;
-        for (uint64_t i = 0; i < valid; i++) {
-            volatile A next = run + A(t[i]);
-            run = next;
-            part[i] = run;
-        }
-        for (uint64_t i = valid; i < SEQ_TILE; i++) part[i] = run;
-        out.partials.emplace(b, std::move(part));
-    };
-    return seq_core<Prod, P, A>(env, pr, count, &out.total, out.starts.data(), on_replay, &out.replayed);
+    const SeqScratch sc = SeqScratch::carve(s->scratch.ptr, ntiles, false);
+    rc = seq_launch<Prod, P, A>(s->stream, &s->launches, sc, pr, count);
+    if (rc) return rc;
+    QSLC_CUDA(cudaMemcpyAsync(s->host_pinned, sc.total, 8, cudaMemcpyDeviceToHost, s->stream));
+    QSLC_CUDA(cudaStreamSynchronize(s->stream));
+    *out = *static_cast<double *>(s->host_pinned);
+    return QSLC_OK;
 }
 
-// Sampling: for each uniform, the element whose partial sum is the first to
-// reach it.  `host_index` maps an element to its basis index for shots that
-// land in replayed tiles.  Outcomes go to out[0..n) in the order of u.
+// Sampling: for each uniform, the basis index of the element whose partial
+// sum is the first to reach it, into out[0..n) in the order of u.
 // strict (sampleAll2, measure.cpp:237-267): the first element whose
 // partial sum exceeds u; a uniform at or above the total lands nowhere and
 // is reported as ~0.  Otherwise (sampleAll): the first partial sum >= u,
 // and 0 above the total.
-template <class Prod, class P, class A, class HostIndex>
-int seq_sample(qslc_state *s, const Prod &pr, uint64_t count, const double *u, uint64_t n,
-               uint64_t *out, HostIndex host_index, bool strict = false)
+template <class Prod, class P, class A>
+int seq_sample(qslc_state *s, const Prod &pr, uint64_t count, const double *u, uint64_t n, uint64_t *out,
+               bool strict = false)
 {
-    SeqOut<A> so;
-    int rc = seq_run<Prod, P, A>(s, pr, count, true, so);
+    const uint64_t ntiles = (count + SEQ_TILE - 1) / SEQ_TILE;
+    int rc = s->scratch.ensure(SeqScratch::carve(nullptr, ntiles, true).bytes);
+    if (!rc) rc = s->scratch2.ensure(2 * SeqScratch::align(n * 8));
     if (rc) return rc;
-    const uint64_t ntiles = so.starts.size();
-    std::vector<uint32_t> order(n);
-    for (uint64_t i = 0; i < n; i++) order[i] = uint32_t(i);
-    std::sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return u[a] < u[b]; });
-    std::vector<double> us(n);
-    for (uint64_t i = 0; i < n; i++) us[i] = u[order[i]];
-
-    std::vector<ResolveItem> items;
-    std::vector<uint64_t> res(n, 0);
-    std::vector<char> on_device(n, 0);
-    uint64_t b = 0;
-    for (uint64_t k = 0; k < n;) {
-        const double uk = us[k];
-        const uint64_t none = strict ? ~uint64_t(0) : 0;
-        auto reaches = [strict](double v, double x) { return strict ? v > x : v >= x; };
-        if (!reaches(double(so.total), uk)) {   // past the total (:167, :258)
-            res[k++] = none;
-            continue;
-        }
-        // first tile whose end reaches uk
-        while (b < ntiles) {
-            double end = (b + 1 < ntiles) ? double(so.starts[b + 1]) : double(so.total);
-            if (reaches(end, uk)) break;
-            b++;
-        }
-        if (b >= ntiles) { res[k++] = none; continue; }
-        const double end = (b + 1 < ntiles) ? double(so.starts[b + 1]) : double(so.total);
-        uint64_t k1 = k;
-        while (k1 < n && reaches(end, us[k1])) k1++;
-        auto pit = so.partials.find(b);
-        if (pit != so.partials.end()) {
-            const std::vector<A> &part = pit->second;
-            for (uint64_t q = k; q < k1; q++) {
-                const double x = us[q];
-                uint64_t i = uint64_t(std::find_if(part.begin(), part.end(),
-                                                   [&](A v) { return reaches(double(v), x); }) -
-                                      part.begin());
-                if (i >= SEQ_TILE) i = SEQ_TILE - 1;
-                res[q] = host_index(b * SEQ_TILE + i);
-            }
-        } else {
-            ResolveItem it{};
-            it.tile = b;
-            it.start = double(so.starts[b]);
-            it.binade = so.guess[b];
-            it.shot0 = uint32_t(k);
-            it.nshot = uint32_t(k1 - k);
-            it.strict = strict ? 1u : 0u;
-            items.push_back(it);
-            for (uint64_t q = k; q < k1; q++) on_device[q] = 1;
-        }
-        k = k1;
-    }
-    if (!items.empty()) {
-        const size_t need = SeqScratch::align(n * 8) * 2 + SeqScratch::align(items.size() * sizeof(ResolveItem));
-        rc = s->scratch2.ensure(need);
-        if (rc) return rc;
-        char *p = static_cast<char *>(s->scratch2.ptr);
-        double *d_u = reinterpret_cast<double *>(p);
-        uint64_t *d_out = reinterpret_cast<uint64_t *>(p + SeqScratch::align(n * 8));
-        ResolveItem *d_items = reinterpret_cast<ResolveItem *>(p + 2 * SeqScratch::align(n * 8));
-        cudaStream_t str = s->stream;
-        QSLC_CUDA(cudaMemcpyAsync(d_u, us.data(), n * 8, cudaMemcpyHostToDevice, str));
-        QSLC_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(ResolveItem),
-                                  cudaMemcpyHostToDevice, str));
-        const unsigned grid = unsigned(std::min<size_t>(items.size(), size_t(sm_count()) * 4));
-        k_seq_resolve<Prod, A><<<grid, SEQ_TPB, 0, str>>>(pr, count, d_items, int(items.size()), d_u, d_out);
-        s->launches++;
-        QSLC_CUDA(cudaGetLastError());
-        std::vector<uint64_t> dev(n);
-        QSLC_CUDA(cudaMemcpyAsync(dev.data(), d_out, n * 8, cudaMemcpyDeviceToHost, str));
-        QSLC_CUDA(cudaStreamSynchronize(str));
-        for (uint64_t q = 0; q < n; q++)
-            if (on_device[q]) res[q] = dev[q];
-    }
-    for (uint64_t q = 0; q < n; q++) out[order[q]] = res[q];
+    const SeqScratch sc = SeqScratch::carve(s->scratch.ptr, ntiles, true);
+    double *d_u = static_cast<double *>(s->scratch2.ptr);
+    uint64_t *d_out = reinterpret_cast<uint64_t *>(static_cast<char *>(s->scratch2.ptr) + SeqScratch::align(n * 8));
+    QSLC_CUDA(cudaMemcpyAsync(d_u, u, n * 8, cudaMemcpyHostToDevice, s->stream));
+    rc = seq_launch<Prod, P, A>(s->stream, &s->launches, sc, pr, count);
+    if (rc) return rc;
+    k_seq_shots<Prod, A><<<unsigned((n + SEQ_TPB / 32 - 1) / (SEQ_TPB / 32)), SEQ_TPB, 0, s->stream>>>(
+        pr, count, ntiles, sc.starts, sc.inside, sc.pieces, sc.total, d_u, uint32_t(n), strict ? 1 : 0, d_out);
+    s->launches++;
+    QSLC_CUDA(cudaGetLastError());
+    QSLC_CUDA(cudaMemcpyAsync(out, d_out, n * 8, cudaMemcpyDeviceToHost, s->stream));
+    QSLC_CUDA(cudaStreamSynchronize(s->stream));
     return QSLC_OK;
 }
 
