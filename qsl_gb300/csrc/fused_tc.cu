@@ -11,11 +11,19 @@
 // x = hi + lo with hi, lo TF32, and D = A_hi B_hi + A_hi B_lo + A_lo B_hi
 // (the A_lo B_lo term is below FP32 resolution).
 //
-// Shared-memory operands use the canonical K-major layout without swizzle:
-// core matrices of 8 rows x 16 bytes, 128 contiguous bytes each, ordered
-// K-chunk fastest then 8-row group; the descriptors' leading byte offset is
-// the step between K-adjacent core matrices (128 B) and the stride byte
-// offset the step between 8-row groups (K/4 * 128 B).
+// A lives in tensor memory (row i in lane i, one 32-bit column per K entry):
+// a thread's group is its lane's row, so the split goes there straight from
+// registers.  From shared memory, writing the two halves of A and reading
+// them twice for the MMAs took more than half of the SM's 128 bytes a clock,
+// and the tiles left 34 KB of L1 for loads in flight: 3.44 ms a block of a
+// 30-qubit state (5.0 TB/s) against 2.61 ms (6.6 TB/s) now, of which 0.54 ms
+// come from loading two tiles ahead instead of one.
+//
+// B uses the canonical K-major shared-memory layout without swizzle: core
+// matrices of 8 rows x 16 bytes, 128 contiguous bytes each, ordered K-chunk
+// fastest then 8-row group; the descriptors' leading byte offset is the step
+// between K-adjacent core matrices (128 B) and the stride byte offset the step
+// between 8-row groups (K/4 * 128 B).
 //
 // Every wait is bounded: if the MMA completion never arrives the kernel
 // records an error code, releases its tensor memory and returns.
@@ -31,9 +39,11 @@ constexpr int TC_M = 128;   // groups per tile
 constexpr int TC_N = 64;
 constexpr int TC_K = 64;
 constexpr int CORE_BYTES = 128;
-constexpr int A_BYTES = TC_M * TC_K * 4;     // 32 KB per split half
 constexpr int B_BYTES = TC_N * TC_K * 4;     // 16 KB per split half
-constexpr uint32_t TMEM_COLS = 64;
+// Tensor memory of a CTA: A_hi, A_lo and D, one 32-bit column per K or N.
+constexpr uint32_t TMEM_COLS = 256, TM_HI = 0, TM_LO = TC_K, TM_D = 2 * TC_K;
+constexpr int ROW_BYTES = 8 * 32 + 16;       // a group's amplitudes in shared memory; 16 bytes keep rows apart
+constexpr int TILE_BYTES = TC_M * ROW_BYTES;
 constexpr long long WAIT_LIMIT = 1ll << 26;
 
 __device__ __forceinline__ uint32_t core_offset(int row, int k)
@@ -63,20 +73,24 @@ __device__ __forceinline__ uint32_t to_tf32(float x)
     return r;
 }
 
-// TF32 split of four consecutive K entries of one row: x = hi + lo.
-__device__ __forceinline__ void split4(float4 x, uint4 &hi, uint4 &lo)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16])
 {
-    hi = make_uint4(to_tf32(x.x), to_tf32(x.y), to_tf32(x.z), to_tf32(x.w));
-    lo = make_uint4(to_tf32(x.x - __uint_as_float(hi.x)), to_tf32(x.y - __uint_as_float(hi.y)),
-                    to_tf32(x.z - __uint_as_float(hi.z)), to_tf32(x.w - __uint_as_float(hi.w)));
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+        "%12, %13, %14, %15};\n" ::"r"(r[0]),
+        "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+        : "memory");
 }
 
-__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t acc)
+// A from tensor memory (row i in lane i, column k its K entry k), B from shared memory
+__device__ __forceinline__ void mma_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t acc)
 {
     asm volatile(
         "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(acc));
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}\n" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(IDESC), "r"(acc)
+        : "memory");
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase)
@@ -105,23 +119,32 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
 
 // bmat: B_hi then B_lo, each [64 n][64 k] row-major fp32 (tf32 values).
 //
-// Pipeline per tile: the 32 amplitudes of this thread's group wait in
-// registers; they are split into shared memory (16-byte stores, one row of
-// a core matrix each), one thread issues the MMAs, and while they run every
-// thread already loads the next tile's amplitudes into the same registers.
-// Tiles cover disjoint groups, so reading the next tile before the current
-// one is written back is safe.
+// Pipeline per tile: the 32 amplitudes of this thread's group are in registers;
+// they are split into tensor memory, one thread issues the MMAs, and every
+// thread at once loads the tile after the next into the same registers, so two
+// tiles are on their way at any time.  Tiles cover disjoint groups, so reading
+// ahead of the stores is safe.
+//
+// LOW is for blocks with three or four of the lowest four qubits, whose
+// groups lie so close that a warp's access to one amplitude of each takes 32
+// sectors in up to 32 lines: the tile's 4096 amplitudes are copied to shared
+// memory and back in ascending order of their place in memory instead, 256
+// bytes a warp at worst in pieces of 32.  Blocks of a 29-qubit state, us,
+// direct and LOW: qubits 0-4 4214 and 1970, {0, 1, 2, 10, 11} 2590 and 2121, 1-5
+// 2385 and 2095, {0, 1, 10, 11, 12} 1838 and 2114, 2-6 1667 and 2102, 10-14 1378
+// and 2132.
+template <bool LOW>
 __global__ void __launch_bounds__(TC_M) k_dense_tc(float2 *__restrict__ st, uint64_t ngroups,
                                                    const float *__restrict__ bmat, uint4 pos_lo,
                                                    unsigned pos_hi, int *__restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *a_hi = smem, *a_lo = smem + A_BYTES;
-    unsigned char *b_hi = smem + 2 * A_BYTES, *b_lo = b_hi + B_BYTES;
+    unsigned char *b_hi = smem, *b_lo = b_hi + B_BYTES;
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ int arrived;
-    __shared__ uint64_t s_off[32];
+    __shared__ uint64_t s_off[32], s_copy[32];
+    __shared__ uint32_t s_row[32];
     const int tid = threadIdx.x, warp = tid >> 5;
     const unsigned pos[5] = {pos_lo.x, pos_lo.y, pos_lo.z, pos_lo.w, pos_hi};
     if (tid < 32) {
@@ -138,6 +161,7 @@ __global__ void __launch_bounds__(TC_M) k_dense_tc(float2 *__restrict__ st, uint
         *reinterpret_cast<float *>(b_hi + o) = bmat[i];
         *reinterpret_cast<float *>(b_lo + o) = bmat[TC_N * TC_K + i];
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     const uint32_t mbar_s = uint32_t(__cvta_generic_to_shared(&mbar));
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_s));
@@ -153,38 +177,90 @@ __global__ void __launch_bounds__(TC_M) k_dense_tc(float2 *__restrict__ st, uint
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_slot;
-    const uint32_t a_hi_s = uint32_t(__cvta_generic_to_shared(a_hi));
-    const uint32_t a_lo_s = uint32_t(__cvta_generic_to_shared(a_lo));
     const uint32_t b_hi_s = uint32_t(__cvta_generic_to_shared(b_hi));
     const uint32_t b_lo_s = uint32_t(__cvta_generic_to_shared(b_lo));
     const uint64_t ntiles = ngroups / TC_M;
-    auto group_base = [&](uint64_t t) {
-        uint64_t b = t * TC_M + tid;
+    auto group_base = [&](uint64_t t, int row) {
+        uint64_t b = t * TC_M + row;
 #pragma unroll
         for (int j = 0; j < 5; j++) b = insert0(b, pos[j]);
         return b;
     };
-    float2 a[32];
-    uint64_t t = blockIdx.x;
-    if (t < ntiles) {
-        const uint64_t b0 = group_base(t);
+    const uint64_t step = gridDim.x;
+    auto load = [&](float2 (&a)[32], uint64_t t) {
+        if (t >= ntiles) return;
+        const uint64_t b = group_base(t, tid);
 #pragma unroll
-        for (int v = 0; v < 32; v++) a[v] = st[b0 | s_off[v]];
+        for (int v = 0; v < 32; v++) a[v] = st[b | s_off[v]];
+    };
+    // LOW: the tile as TC_M rows in shared memory, two tiles by turns.  Copy i
+    // of a thread is local amplitude 128 i + tid; a tile's 12 bits, ascending,
+    // are each a bit of the row or of the place in it.
+    unsigned char *const rows = smem + 2 * B_BYTES;
+    uint64_t my_off = 0;
+    uint32_t my_row = 0;
+    if constexpr (LOW) {
+        auto place = [&](unsigned l, uint64_t &g, uint32_t &r) {
+            unsigned q = 0, nv = 0, nr = 0;
+            g = 0;
+            r = 0;
+            for (int j = 0; j < 12; j++, q++) {
+                while (nr == 7 && q != pos[nv]) q++;         // 7 row bits found: only the block's are left
+                const bool block = nv < 5 && q == pos[nv];
+                if ((l >> j) & 1) {
+                    g |= uint64_t(1) << q;
+                    r += block ? 8u << nv : uint32_t(ROW_BYTES) << nr;
+                }
+                if (block) nv++;
+                else nr++;
+            }
+        };
+        place(unsigned(tid), my_off, my_row);
+        if (tid < 32) place(unsigned(tid) << 7, s_copy[tid], s_row[tid]);
+        __syncthreads();
     }
-    uint32_t phase = 0;
-    bool ok = true;
-    for (; t < ntiles && ok; t += gridDim.x) {
-        const uint64_t base = group_base(t);
-        // row `tid` of A: K entries 4j..4j+3 are amplitudes 2j, 2j+1 as (re, im)
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            uint4 hi, lo;
-            split4(make_float4(a[2 * j].x, a[2 * j].y, a[2 * j + 1].x, a[2 * j + 1].y), hi, lo);
-            const uint32_t o = core_offset(tid, 4 * j);
-            *reinterpret_cast<uint4 *>(a_hi + o) = hi;
-            *reinterpret_cast<uint4 *>(a_lo + o) = lo;
+    auto copy_in = [&](uint64_t t, int half) {
+        if (t < ntiles) {
+            const float2 *src = st + (group_base(t, 0) | my_off);
+            const uint32_t dst = uint32_t(__cvta_generic_to_shared(rows + half * TILE_BYTES)) + my_row;
+#pragma unroll 8
+            for (int i = 0; i < 32; i++)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + s_row[i]), "l"(src + s_copy[i])
+                             : "memory");
         }
-        asm volatile("fence.proxy.async.shared::cta;");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const uint32_t lanes = tmem + (uint32_t(warp * 32) << 16);   // this warp's rows
+    uint32_t phase = 0;
+    // one tile, whose amplitudes are in `a` (LOW: on their way to rows);
+    // false when the wait ran out
+    auto tile = [&](float2 (&a)[32], uint64_t t, int half) -> bool {
+        unsigned char *const buf = rows + half * TILE_BYTES;
+        if constexpr (LOW) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const float4 x = *reinterpret_cast<const float4 *>(buf + tid * ROW_BYTES + 16 * j);
+                a[2 * j] = make_float2(x.x, x.y);
+                a[2 * j + 1] = make_float2(x.z, x.w);
+            }
+        }
+        const uint64_t base = LOW ? group_base(t, 0) : group_base(t, tid);
+        // row `tid` of A: K entries 2v, 2v + 1 are amplitude v's (re, im)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            uint32_t hi[16], lo[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const float x = i & 1 ? a[8 * c + i / 2].y : a[8 * c + i / 2].x;
+                hi[i] = to_tf32(x);
+                lo[i] = to_tf32(x - __uint_as_float(hi[i]));
+            }
+            tmem_st16(lanes + TM_HI + uint32_t(16 * c), hi);
+            tmem_st16(lanes + TM_LO + uint32_t(16 * c), lo);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -193,51 +269,68 @@ __global__ void __launch_bounds__(TC_M) k_dense_tc(float2 *__restrict__ st, uint
 #pragma unroll
             for (int s = 0; s < TC_K / 8; s++) {       // K = 8 per instruction: two core matrices
                 const uint32_t koff = uint32_t(2 * s * CORE_BYTES);
-                mma_tf32(tmem, smem_desc(a_hi_s + koff), smem_desc(b_hi_s + koff), acc);
+                const uint64_t bh = smem_desc(b_hi_s + koff), bl = smem_desc(b_lo_s + koff);
+                mma_tf32(tmem + TM_D, tmem + TM_HI + 8 * s, bh, acc);
                 acc = 1;
-                mma_tf32(tmem, smem_desc(a_hi_s + koff), smem_desc(b_lo_s + koff), 1);
-                mma_tf32(tmem, smem_desc(a_lo_s + koff), smem_desc(b_hi_s + koff), 1);
+                mma_tf32(tmem + TM_D, tmem + TM_HI + 8 * s, bl, 1);
+                mma_tf32(tmem + TM_D, tmem + TM_LO + 8 * s, bh, 1);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                 mbar_s));
         }
-        // the next tile's amplitudes travel while the MMAs run
-        const uint64_t tn = t + gridDim.x;
-        if (tn < ntiles) {
-            const uint64_t bn = group_base(tn);
-#pragma unroll
-            for (int v = 0; v < 32; v++) a[v] = st[bn | s_off[v]];
-        }
+        // the amplitudes of the tile after the next travel from here on
+        if constexpr (!LOW) load(a, t + 2 * step);
         // one thread polls the barrier (bounded); the block follows its outcome
         if (tid == 0) arrived = mbar_wait(mbar_s, phase) ? 1 : 0;
         __syncthreads();
         if (!arrived) {
-            ok = false;
             if (tid == 0) {
                 atomicExch(err, 1);
                 mbar_wait(mbar_s, phase);            // give work in flight a last bounded wait
             }
-            break;
+            return false;
         }
         phase ^= 1;
         asm volatile("tcgen05.fence::after_thread_sync;");
         // row tid of D: lane tid of tensor memory, 64 fp32 columns
-        const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16);
 #pragma unroll
         for (int c = 0; c < 4; c++) {
             uint32_t r[16];
-            tmem_ld16(taddr + uint32_t(16 * c), r);
+            tmem_ld16(lanes + TM_D + uint32_t(16 * c), r);
             asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int v = 8 * c + i;
-                st[base | s_off[v]] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                const float2 x = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                if constexpr (LOW) *reinterpret_cast<float2 *>(buf + tid * ROW_BYTES + 8 * v) = x;
+                else st[base | s_off[v]] = x;
             }
+        }
+        if constexpr (LOW) {
+            __syncthreads();
+#pragma unroll 8
+            for (int i = 0; i < 32; i++)
+                st[(base | my_off) + s_copy[i]] = *reinterpret_cast<const float2 *>(buf + my_row + s_row[i]);
         }
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;");
+        if constexpr (LOW) copy_in(t + 2 * step, half);
+        return true;
+    };
+    float2 a0[32], a1[32];
+    if constexpr (LOW) {
+        copy_in(blockIdx.x, 0);
+        copy_in(blockIdx.x + step, 1);
+    } else {
+        load(a0, blockIdx.x);
+        load(a1, blockIdx.x + step);
     }
+    for (uint64_t t = blockIdx.x; t < ntiles; t += 2 * step) {
+        if (!tile(a0, t, 0)) break;
+        if (t + step >= ntiles || !tile(LOW ? a0 : a1, t + step, 1)) break;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
@@ -283,16 +376,17 @@ bool tc_usable(const qslc_state *s) { return s->n >= 12; }
 int tc_launch(qslc_state *s, const float *d_b, const unsigned *pos, int *d_err)
 {
     const uint64_t ngroups = uint64_t(1) << (s->n - 5);
-    const int smem = 2 * A_BYTES + 2 * B_BYTES;
-    static bool attr = false;
-    if (!attr) {
-        QSLC_CUDA(cudaFuncSetAttribute(k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr = true;
-    }
     const uint64_t tiles = ngroups / TC_M;
     const unsigned grid = unsigned(std::min<uint64_t>(tiles, uint64_t(sm_count()) * 2));
-    k_dense_tc<<<grid, TC_M, smem, s->stream>>>(static_cast<float2 *>(s->amps), ngroups, d_b,
-                                                make_uint4(pos[0], pos[1], pos[2], pos[3]), pos[4], d_err);
+    auto go = [&](auto *kern, int smem) -> int {
+        QSLC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kern<<<grid, TC_M, smem, s->stream>>>(static_cast<float2 *>(s->amps), ngroups, d_b,
+                                              make_uint4(pos[0], pos[1], pos[2], pos[3]), pos[4], d_err);
+        return QSLC_OK;
+    };
+    const bool low = pos[2] < 4;          // three of the lowest four (positions ascend)
+    const int rc = low ? go(k_dense_tc<true>, 2 * B_BYTES + 2 * TILE_BYTES) : go(k_dense_tc<false>, 2 * B_BYTES);
+    if (rc) return rc;
     s->launches++;
     QSLC_CUDA(cudaGetLastError());
     return QSLC_OK;
