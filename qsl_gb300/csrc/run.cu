@@ -20,7 +20,7 @@
 // instructions: 17 gates of a 25-qubit circuit take 300 us a run, 80 of them
 // the traffic (four such layers: 5.6 ms before, 2.7 ms).  complex128 runs
 // are bound by the FP64 and ALU pipes as the single sweeps are, and gain where
-// launches or moves count: 8 layers of 10 qubits 418 -> 256 us.
+// launches or moves count: 8 layers of 10 qubits 418 -> 203 us.
 #include "gatemath.cuh"
 
 #include <algorithm>
@@ -71,8 +71,10 @@ template <> struct RunCoef<double> {
 };
 static_assert(offsetof(RunCoef<double>, ms) == offsetof(SlowCoef, ms), "SlowCoef heads RunCoef<double>");
 
-// Register bits of a thread: 4 amplitudes of 16 bytes or 16 of 8.
+// Register bits of a thread: 4 amplitudes of 16 bytes or 16 of 8, and on small
+// states 2 of 16 bytes or 4 of 8 (reg_bits).
 template <class T> constexpr int REG_BITS = sizeof(T) == 8 ? 2 : 4;
+template <class T> constexpr int SMALL_REG_BITS = sizeof(T) == 8 ? 1 : 2;
 
 template <class T, int NG>
 struct RunArgs {
@@ -97,23 +99,25 @@ __device__ __forceinline__ uint32_t slot_of(uint32_t l)
     else return l ^ ((l >> 4) & 15u);
 }
 
-// ---- complex128: 4 amplitudes ------------------------------------------------
+// ---- complex128: 2 or 4 amplitudes -------------------------------------------
 
-template <int OP>
-__device__ __forceinline__ void run_pairs(double2 &x0, double2 &x1, double2 &y0, double2 &y1, unsigned set,
-                                          const Coef<double> &k, const SlowCoef *q, const emu::DivConst *kd)
+template <int OP, int A>
+__device__ __forceinline__ void run_pairs(double2 (&v)[A], unsigned set, const Coef<double> &k, const SlowCoef *q,
+                                          const emu::DivConst *kd)
 {
     auto pair = [&](double2 &a0, double2 &a1) {
         if constexpr (OP == P_SWAP || OP == P_Y) pair_update<double, OP>(a0, a1, k);
         else pair_either<OP>(a0, a1, k, q, kd);
     };
-    if (set == 3) {
-        pair(x0, x1);
-        pair(y0, y1);
+    if constexpr (A == 2) {
+        pair(v[0], v[1]);
+    } else if (set == 3) {
+        pair(v[0], v[1]);
+        pair(v[2], v[3]);
     } else if (set == 1) {
-        pair(x0, x1);
+        pair(v[0], v[1]);
     } else {
-        pair(y0, y1);
+        pair(v[2], v[3]);
     }
 }
 
@@ -122,8 +126,8 @@ __device__ __forceinline__ void run_rotate(double2 &a, uint32_t flip, const Coef
     if (!phase_flip_lean(a, flip, k)) a = flip ? phase_slow<true>(a, q) : phase_slow<false>(a, q);
 }
 
-template <int NG>
-__device__ __forceinline__ void run_gate(double2 (&v)[4], const RunGate &g, const RunCoef<double> &r, bool flip_all,
+template <int A, int NG>
+__device__ __forceinline__ void run_gate(double2 (&v)[A], const RunGate &g, const RunCoef<double> &r, bool flip_all,
                                          const RunArgs<double, NG> &a)
 {
     Coef<double> k{};
@@ -135,39 +139,39 @@ __device__ __forceinline__ void run_gate(double2 (&v)[4], const RunGate &g, cons
     const SlowCoef *q = reinterpret_cast<const SlowCoef *>(&r);
     if (g.op >= RUN_NEG) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
+        for (int i = 0; i < A; i++) {
             if (!((g.set >> i) & 1)) continue;
             if (g.op == RUN_NEG) diag_update<double, D_NEG>(v[i], k);
             else run_rotate(v[i], (((g.neg >> i) & 1) != 0) != flip_all ? 0x80000000u : 0u, k, q);
         }
         return;
     }
-    if (g.p) {
-        const double2 m = v[1];
-        v[1] = v[2];
-        v[2] = m;
-    }
+    auto turn = [&] {
+        if constexpr (A == 4)
+            if (g.p) {
+                const double2 m = v[1];
+                v[1] = v[2];
+                v[2] = m;
+            }
+    };
+    turn();
     switch (g.op) {
-    case RUN_SWAP: run_pairs<P_SWAP>(v[0], v[1], v[2], v[3], g.set, k, q, &a.h.kd); break;
-    case RUN_Y: run_pairs<P_Y>(v[0], v[1], v[2], v[3], g.set, k, q, &a.h.kd); break;
-    case RUN_H: run_pairs<P_H>(v[0], v[1], v[2], v[3], g.set, k, q, &a.h.kd); break;
-    case RUN_RX: run_pairs<P_RX>(v[0], v[1], v[2], v[3], g.set, k, q, &a.h.kd); break;
-    default: run_pairs<P_RY>(v[0], v[1], v[2], v[3], g.set, k, q, &a.h.kd); break;
+    case RUN_SWAP: run_pairs<P_SWAP>(v, g.set, k, q, &a.h.kd); break;
+    case RUN_Y: run_pairs<P_Y>(v, g.set, k, q, &a.h.kd); break;
+    case RUN_H: run_pairs<P_H>(v, g.set, k, q, &a.h.kd); break;
+    case RUN_RX: run_pairs<P_RX>(v, g.set, k, q, &a.h.kd); break;
+    default: run_pairs<P_RY>(v, g.set, k, q, &a.h.kd); break;
     }
-    if (g.p) {
-        const double2 m = v[1];
-        v[1] = v[2];
-        v[2] = m;
-    }
+    turn();
 }
 
-// ---- complex64: 16 amplitudes ------------------------------------------------
+// ---- complex64: 4 or 16 amplitudes -------------------------------------------
 
-template <int OP, int P, bool ALL>
-__device__ __forceinline__ void run_pairs16(float2 (&v)[16], unsigned set, const Coef<float> &k, float hinv)
+template <int OP, int P, bool ALL, int A>
+__device__ __forceinline__ void run_pairs_on(float2 (&v)[A], unsigned set, const Coef<float> &k, float hinv)
 {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < A / 2; i++) {
         const int i0 = ((i >> P) << (P + 1)) | (i & ((1 << P) - 1)), i1 = i0 | (1 << P);
         if (!ALL && !((set >> i) & 1)) continue;
         if constexpr (OP == P_H) {
@@ -190,24 +194,29 @@ __device__ __forceinline__ void run_pairs16(float2 (&v)[16], unsigned set, const
     }
 }
 
-template <int OP, bool ALL>
-__device__ __forceinline__ void run_pairs_at(float2 (&v)[16], int p, unsigned set, const Coef<float> &k, float hinv)
+template <int OP, bool ALL, int A>
+__device__ __forceinline__ void run_pairs_at(float2 (&v)[A], int p, unsigned set, const Coef<float> &k, float hinv)
 {
-    switch (p) {
-    case 0: run_pairs16<OP, 0, ALL>(v, set, k, hinv); break;
-    case 1: run_pairs16<OP, 1, ALL>(v, set, k, hinv); break;
-    case 2: run_pairs16<OP, 2, ALL>(v, set, k, hinv); break;
-    default: run_pairs16<OP, 3, ALL>(v, set, k, hinv); break;
+    if constexpr (A == 4) {
+        if (p == 0) run_pairs_on<OP, 0, ALL>(v, set, k, hinv);
+        else run_pairs_on<OP, 1, ALL>(v, set, k, hinv);
+    } else {
+        switch (p) {
+        case 0: run_pairs_on<OP, 0, ALL>(v, set, k, hinv); break;
+        case 1: run_pairs_on<OP, 1, ALL>(v, set, k, hinv); break;
+        case 2: run_pairs_on<OP, 2, ALL>(v, set, k, hinv); break;
+        default: run_pairs_on<OP, 3, ALL>(v, set, k, hinv); break;
+        }
     }
 }
 
-template <bool ALL>
-__device__ __forceinline__ void run_rotate16(float2 (&v)[16], unsigned set, unsigned neg, bool flip_all,
+template <bool ALL, int A>
+__device__ __forceinline__ void run_rotate_on(float2 (&v)[A], unsigned set, unsigned neg, bool flip_all,
                                              const Coef<float> &k)
 {
     const float sp = flip_all ? -k.s : k.s;
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
+    for (int i = 0; i < A; i++) {
         if (!ALL && !((set >> i) & 1)) continue;
         const float s = ((neg >> i) & 1) ? -sp : sp;
         const float x = v[i].x, y = v[i].y;
@@ -216,14 +225,14 @@ __device__ __forceinline__ void run_rotate16(float2 (&v)[16], unsigned set, unsi
     }
 }
 
-template <int NG>
-__device__ __forceinline__ void run_gate(float2 (&v)[16], const RunGate &g, const RunCoef<float> &r, bool flip_all,
+template <int A, int NG>
+__device__ __forceinline__ void run_gate(float2 (&v)[A], const RunGate &g, const RunCoef<float> &r, bool flip_all,
                                          const RunArgs<float, NG> &a)
 {
     Coef<float> k{};
     k.c = g.op == RUN_H ? a.h.c : r.c;
     k.s = r.s;
-    const bool all = g.set == 0xFF;
+    const bool all = g.set == (1u << (A / 2)) - 1u;
     switch (g.op) {
     case RUN_SWAP: run_pairs_at<P_SWAP, false>(v, g.p, g.set, k, 0.f); break;
     case RUN_Y: run_pairs_at<P_Y, false>(v, g.p, g.set, k, 0.f); break;
@@ -241,22 +250,22 @@ __device__ __forceinline__ void run_gate(float2 (&v)[16], const RunGate &g, cons
         break;
     case RUN_NEG:
 #pragma unroll
-        for (int i = 0; i < 16; i++)
+        for (int i = 0; i < A; i++)
             if ((g.set >> i) & 1) diag_update<float, D_NEG>(v[i], k);
         break;
     default:
-        if (g.set == 0xFFFF) run_rotate16<true>(v, g.set, g.neg, flip_all, k);
-        else run_rotate16<false>(v, g.set, g.neg, flip_all, k);
+        if (g.set == (1u << A) - 1u) run_rotate_on<true>(v, g.set, g.neg, flip_all, k);
+        else run_rotate_on<false>(v, g.set, g.neg, flip_all, k);
         break;
     }
 }
 
-template <class T, class IX, int NG>
+template <class T, class IX, int NG, int R>
 __global__ void __launch_bounds__(256, RUN_CTAS)
     k_run(cplx<T> *__restrict__ st, const __grid_constant__ RunArgs<T, NG> a)
 {
     extern __shared__ __align__(128) unsigned char run_smem[];
-    constexpr int R = REG_BITS<T>, A = 1 << R;
+    constexpr int A = 1 << R;
     constexpr uint32_t AB = sizeof(cplx<T>);
     auto at = [&](uint32_t byte) -> cplx<T> & { return *reinterpret_cast<cplx<T> *>(run_smem + byte); };
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
@@ -328,17 +337,32 @@ struct Shape {
     unsigned bits, low, threads;
 };
 
+// The register bits of a thread.  A small state leaves most of the chip idle,
+// and a gate takes the time that one warp needs for its amplitudes, about 8
+// clocks an instruction: fewer amplitudes a thread, in more warps, are quicker
+// although the targets of a run then take more steps.  Circuits of 8 layers, us,
+// usual and small: complex128 of 6 qubits 166 and 135, of 10 258 and 225, of 14
+// 308 and 255, of 17 384 and 317 (to 19 qubits, where runs_any ends); complex64 of 6 qubits 121 and 107, of 12 235
+// and 216, of 14 228 and 232.
+template <class T> constexpr unsigned SMALL_STATE = sizeof(T) == 8 ? 19 : 13;
+template <class T> int reg_bits(const qslc_state *s)
+{
+    return s->n <= SMALL_STATE<T> ? SMALL_REG_BITS<T> : REG_BITS<T>;
+}
+
 // Small states take small tiles: many CTAs share the arithmetic, which a run
 // of few gates does not fill otherwise.  Circuits of 8 layers on one GB300,
-// us, tiles of 2^8 / 2^9 / 2^10 / 2^11 amplitudes: complex128 of 10 qubits
-// 248 / 256 / 284 / 284, of 14 342 / 341 / 365 / 515, of 17 433 / 428 / 445 /
-// 636; complex64 of 10 qubits 204 / 211 / 195 / -, of 25 (4 layers) - / - /
-// 3044 / 2871 and 2655 with 2^12.  Two contiguous low qubits were never slower
-// than three or four: the others are left to the run.
+// us, tiles of 2^7 / 2^8 / 2^9 / 2^10 amplitudes: complex128 of 10 qubits 229 /
+// 217 / 225 / 297, of 14 261 / 248 / 255 / 355, of 17 329 / 316 / 317 / 437;
+// complex64 of 10 qubits 217 / 192 / 196 / 186, of 14 256 / 230 / 232 / 219,
+// of 25 (4 layers) 3044 with 2^10, 2871 with 2^11 and 2655 with 2^12.  Two
+// contiguous low qubits were never slower than three or four: the others are
+// left to the run.
 Shape shape_of(const qslc_state *s)
 {
-    const unsigned b = std::min(s->dtype == QSLC_C128 ? (s->n >= 18 ? 11u : 9u) : (s->n >= 20 ? 12u : 10u), s->n);
-    const unsigned r = s->dtype == QSLC_C128 ? REG_BITS<double> : REG_BITS<float>;
+    const bool dbl = s->dtype == QSLC_C128;
+    const unsigned b = std::min(dbl ? (s->n > SMALL_STATE<double> ? 11u : 8u) : (s->n >= 20 ? 12u : 10u), s->n);
+    const unsigned r = unsigned(dbl ? reg_bits<double>(s) : reg_bits<float>(s));
     const unsigned t = b >= r + 8 ? 256 : b > r + 5 ? 1u << (b - r) : 32;
     return Shape{b, std::min(b, 2u), std::min(t, 1u << b)};
 }
@@ -421,10 +445,10 @@ bool is_diagonal(RunOp op) { return op >= RUN_NEG; }
 // The kernel's view of gate o in a step with register bits `reg` (state
 // qubits; reg[i] is register bit i) of a tile whose qubits' local numbers are
 // `local` (0xFF: not in the tile).
-template <class T>
+template <class T, int R>
 RunGate encode(const Lowered<T> &o, const unsigned *reg, const uint8_t *local)
 {
-    constexpr int R = REG_BITS<T>, A = 1 << R;
+    constexpr int A = 1 << R;
     RunGate g{};
     g.op = o.op;
     auto reg_bit = [&](unsigned q) {
@@ -465,7 +489,7 @@ RunGate encode(const Lowered<T> &o, const unsigned *reg, const uint8_t *local)
     return g;
 }
 
-template <class T, int NG>
+template <class T, int NG, int R>
 int launch_run_t(qslc_state *s, const std::vector<Lowered<T>> &ops, uint64_t mask)
 {
     const Shape sh = shape_of(s);
@@ -494,7 +518,6 @@ int launch_run_t(qslc_state *s, const std::vector<Lowered<T>> &ops, uint64_t mas
     a.h = hcoef;
     a.hinv = 1.0f / float(hcoef.c);
     a.nsteps = 0;
-    constexpr int R = REG_BITS<T>;
     for (size_t i = 0; i < ops.size();) {
         // as many gates as have their targets in R register bits
         unsigned reg[R];
@@ -526,7 +549,7 @@ int launch_run_t(qslc_state *s, const std::vector<Lowered<T>> &ops, uint64_t mas
         sp.count = uint8_t(j - i);
         for (int k = 0; k < R; k++) sp.bit[k] = local[reg[k]];
         for (; i < j; i++) {
-            a.gate[i] = encode<T>(ops[i], reg, local);
+            a.gate[i] = encode<T, R>(ops[i], reg, local);
             a.coef[i] = ops[i].coef;
         }
     }
@@ -534,7 +557,7 @@ int launch_run_t(qslc_state *s, const std::vector<Lowered<T>> &ops, uint64_t mas
     const size_t smem = sizeof(cplx<T>) << sh.bits;
     auto go = [&](auto ix) -> int {
         using IX = decltype(ix);
-        auto *kern = k_run<T, IX, NG>;
+        auto *kern = k_run<T, IX, NG, R>;
         static std::atomic<int> per_sm[RUN_MAX_BITS + 1] = {};
         if (!per_sm[sh.bits]) {
             QSLC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -548,7 +571,9 @@ int launch_run_t(qslc_state *s, const std::vector<Lowered<T>> &ops, uint64_t mas
         kern<<<unsigned(grid), sh.threads, smem, s->stream>>>(static_cast<cplx<T> *>(s->amps), a);
         return QSLC_OK;
     };
-    const int rc = s->n <= 31 ? go(uint32_t(0)) : go(uint64_t(0));
+    int rc;
+    if constexpr (R == SMALL_REG_BITS<T>) rc = go(uint32_t(0));
+    else rc = s->n <= 31 ? go(uint32_t(0)) : go(uint64_t(0));
     if (rc) return rc;
     s->launches++;
     QSLC_CUDA(cudaGetLastError());
@@ -560,7 +585,11 @@ int launch_run(qslc_state *s, const std::vector<GateOp> &gates, uint64_t mask)
 {
     std::vector<Lowered<T>> ops;
     for (const GateOp &g : gates) lower<T>(g, ops);
-    return ops.size() <= 16 ? launch_run_t<T, 16>(s, ops, mask) : launch_run_t<T, RUN_MAX_GATES>(s, ops, mask);
+    if (reg_bits<T>(s) == SMALL_REG_BITS<T>)
+        return ops.size() <= 16 ? launch_run_t<T, 16, SMALL_REG_BITS<T>>(s, ops, mask)
+                                : launch_run_t<T, RUN_MAX_GATES, SMALL_REG_BITS<T>>(s, ops, mask);
+    return ops.size() <= 16 ? launch_run_t<T, 16, REG_BITS<T>>(s, ops, mask)
+                            : launch_run_t<T, RUN_MAX_GATES, REG_BITS<T>>(s, ops, mask);
 }
 
 // The qubits a gate needs in the tile: those along which it mixes amplitudes.
@@ -601,10 +630,11 @@ bool is_move(int code)
 // enough for launches to count more than arithmetic.  On larger ones the
 // arithmetic binds, and a rotation takes 1.71 clocks per amplitude and SM in a
 // run (coefficients read per gate, a barrier per two gates) against 1.29 in
-// k_group2.  Circuits of 8 layers, us, runs against pairs: 17 qubits 445 and
-// 746, 18 qubits 799 and 845, 20 qubits (20 layers) 3494 and 3721, there with
-// runs of moves beside the pairs 3134.
-bool runs_any(const qslc_state *s) { return s->dtype == QSLC_C64 || s->n <= 17; }
+// k_group2.  Circuits of 8 layers, us, pairs with runs of moves beside them
+// against runs of everything: of rotations and all two-qubit gates, 18 qubits
+// 702 and 462, 19 qubits 949 and 785; of rotations and controlNots, 18 qubits
+// 591 and 460, 19 qubits 852 and 822, 20 qubits 1231 and 1514.
+bool runs_any(const qslc_state *s) { return s->dtype == QSLC_C64 || s->n <= SMALL_STATE<double>; }
 
 // Whether one run is quicker than the gates' own sweeps, by the share of the
 // state that each moves (in quarters of a read and write of all of it) and,

@@ -92,3 +92,15 @@ def test_runs_of_moves_on_large_states(qsl, n):
     b, alone = run(qsl, st, circ, True)
     assert np.array_equal(bits(a), bits(b))
     assert held < alone
+
+
+@pytest.mark.parametrize("n, dtype", [(n, np.complex128) for n in (7, 12, 17, 19)] + [(n, np.complex64) for n in (7, 12, 14)])
+def test_runs_around_the_small_register_form(qsl, n, dtype):
+    # complex128 states of at most 19 qubits and complex64 ones of at most 13 keep fewer amplitudes a thread
+    rng = np.random.default_rng(300 + n)
+    st = random_state(rng, n, dtype)
+    circ = gates(rng, n, 120)
+    a, held = run(qsl, st, circ, False)
+    b, alone = run(qsl, st, circ, True)
+    assert np.array_equal(bits(a), bits(b))
+    assert held < alone
