@@ -111,6 +111,34 @@ QSLC_HD bool easy_range(uint64_t a)
 }
 QSLC_HD bool easy_product(uint64_t a) { return easy_range(a) & (uint32_t(a) != 0); }
 
+// ---- squares ------------------------------------------------------------------
+// m * m of a significand m lies in [2^104, 2^106).  It is half-way between two
+// doubles only when it has 51 or 52 trailing zeros, m then 26: an operand with
+// one of its low 25 bits set rounds on the next bit alone.  The exponent field
+// is 512 to 1533, so that the square is normal.
+QSLC_HD bool easy_square(uint64_t a)
+{
+    const uint32_t h = uint32_t(a >> 32) & 0x7FFFFFFFu;
+    return ((h - (512u << 20)) < (1022u << 20)) & ((uint32_t(a) & 0x1FFFFFFu) != 0);
+}
+
+// The bits of RN(a * a).
+QSLC_HD uint64_t lean_square(uint64_t a)
+{
+    const uint32_t h = uint32_t(a >> 32) & 0x7FFFFFFFu;
+    const uint32_t ml = uint32_t(a), mh = (h & 0xFFFFFu) | 0x100000u;
+    const uint64_t t0 = uint64_t(ml) * ml;
+    const uint64_t t1 = uint64_t(ml) * (2 * mh) + (t0 >> 32);
+    const uint64_t t2 = uint64_t(mh) * mh + (t1 >> 32);          // t2 : low word of t1 : low word of t0
+    const uint32_t top = uint32_t(t2 >> 41);                     // 1: from 2^105 up
+    const uint32_t left = 12 - top, w1 = uint32_t(t1), w0 = uint32_t(t0);
+    const uint64_t sig = (t2 << left) | (w1 >> (32 - left));
+    const uint32_t half = ((w1 << left) | (w0 >> (32 - left))) >> 31;
+    // exponent field 2 E - 1023 + top, less one for the hidden bit
+    const uint32_t ex = ((h & 0x7FF00000u) << 1) - (1024u << 20) + (top << 20);
+    return sig + (uint64_t(ex) << 32) + half;
+}
+
 // (r2:r1:r0) + (k:s1:s0), the top two words: one carry chain.
 QSLC_HD uint64_t round96(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t s0, uint32_t s1, uint32_t k, uint32_t &rest)
 {

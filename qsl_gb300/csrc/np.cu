@@ -264,10 +264,16 @@ struct ProdNPMask {
     unsigned t;
     uint32_t o;
     __device__ __forceinline__ uint64_t index(uint64_t j) const { return basis[j]; }
+    __device__ __forceinline__ cplx<T> amp(uint64_t j) const
+    {
+        cplx<T> a;
+        a.x = a.y = T(0);
+        if (((basis[j] >> t) & 1u) == o) a = amps[j];
+        return a;
+    }
     __device__ __forceinline__ T p(uint64_t j) const
     {
-        if (((basis[j] >> t) & 1u) != o) return T(0);
-        cplx<T> a = amps[j];
+        const cplx<T> a = amp(j);
         return norm2_rn(a.x, a.y);
     }
 };
@@ -276,9 +282,10 @@ struct ProdNPAll {
     const cplx<T> *amps;
     const uint32_t *basis;
     __device__ __forceinline__ uint64_t index(uint64_t j) const { return basis[j]; }
+    __device__ __forceinline__ cplx<T> amp(uint64_t j) const { return amps[j]; }
     __device__ __forceinline__ T p(uint64_t j) const
     {
-        cplx<T> a = amps[j];
+        const cplx<T> a = amp(j);
         return norm2_rn(a.x, a.y);
     }
 };

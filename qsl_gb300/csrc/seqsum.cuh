@@ -31,6 +31,7 @@
 #include <cmath>
 #include <vector>
 
+#include "lean.cuh"
 #include "qslc_internal.cuh"
 #include "replay.cuh"
 
@@ -39,6 +40,7 @@ namespace qslc {
 constexpr int SEQ_TILE = 4096;
 constexpr int SEQ_TPB = 256;
 constexpr int SEQ_PER = SEQ_TILE / SEQ_TPB;
+constexpr int SEQ_AHEAD = 4;               // terms a thread of k_seq_steps loads together
 constexpr int SEQ_PIECES = SEQ_TPB / 32;   // pieces of a tile: a warp's terms
 constexpr int SEQ_PIECE = SEQ_TILE / SEQ_PIECES;
 
@@ -51,9 +53,10 @@ struct ProdHalf {        // amplitudes with bit t == outcome, ascending
     unsigned t;
     uint64_t obit;
     __device__ __forceinline__ uint64_t index(uint64_t j) const { return insert0(j, t) | obit; }
+    __device__ __forceinline__ cplx<T> amp(uint64_t j) const { return amps[index(j)]; }
     __device__ __forceinline__ T p(uint64_t j) const
     {
-        cplx<T> a = amps[index(j)];
+        const cplx<T> a = amp(j);
         return norm2_rn(a.x, a.y);
     }
 };
@@ -62,12 +65,45 @@ template <class T>
 struct ProdAll {         // every amplitude, ascending
     const cplx<T> *amps;
     __device__ __forceinline__ uint64_t index(uint64_t j) const { return j; }
+    __device__ __forceinline__ cplx<T> amp(uint64_t j) const { return amps[j]; }
     __device__ __forceinline__ T p(uint64_t j) const
     {
-        cplx<T> a = amps[j];
+        const cplx<T> a = amp(j);
         return norm2_rn(a.x, a.y);
     }
 };
+
+// |a|^2 of N amplitudes a thread, RN(RN(x x) + RN(y y)); all lanes call it.
+// complex128: the FP64 pipe alone would take three operations a term.  A warp
+// whose parts are all easy (lean.cuh) takes squares on the integer pipes, about
+// 20 instructions each.  k_seq_steps leaves the pipe the other square and the
+// sum (BOTH false): with the sum alone its ALU pipe, which counts the grid steps,
+// is 80% busy and the FP64 pipe 31%.  Over all 2^28 amplitudes 740 us with no
+// square on the integer pipes, 660 with both, 608 with one.  The walk, one CTA
+// that waits for its terms, leaves the sum alone: 138 -> 126 us at 20 qubits.
+template <bool BOTH, int N>
+__device__ __forceinline__ void norms(const float2 (&a)[N], float (&p)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) p[i] = norm2_rn(a[i].x, a[i].y);
+}
+template <bool BOTH, int N>
+__device__ __forceinline__ void norms(const double2 (&a)[N], double (&p)[N])
+{
+    auto bits = [](double v) { return uint64_t(__double_as_longlong(v)); };
+    auto square = [&](double v) { return __longlong_as_double((long long)emu::lean_square(bits(v))); };
+    bool easy = true;
+#pragma unroll
+    for (int i = 0; i < N; i++) easy &= emu::easy_square(bits(a[i].x)) & (!BOTH || emu::easy_square(bits(a[i].y)));
+    if (__all_sync(0xffffffffu, easy)) {
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            p[i] = __dadd_rn(square(a[i].x), BOTH ? square(a[i].y) : __dmul_rn(a[i].y, a[i].y));
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i++) p[i] = norm2_rn(a[i].x, a[i].y);
+    }
+}
 
 // ---------------------------------------------------------------------------
 // Scans of transducers.
@@ -306,12 +342,16 @@ __global__ void __launch_bounds__(SEQ_TPB, 4) k_seq_steps(Prod pr, uint64_t coun
                                                           uint64_t *__restrict__ steps, uint64_t *__restrict__ pieces,
                                                           uint8_t *__restrict__ flags, double *__restrict__ est)
 {
-    __shared__ Tx ptx[SEQ_PIECES];
+    // of this tile and the one before, which thread 0 may still be at
+    __shared__ Tx ptxs[2][SEQ_PIECES];
+    __shared__ unsigned seen[2][SEQ_PIECES];
     __shared__ double psum[SEQ_PIECES];
     constexpr uint64_t CAP = uint64_t(1) << (fp_traits<A>::MANT + 1);
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t todo = redo ? redo[0] : ntiles;
-    for (uint64_t i = blockIdx.x; i < todo; i += gridDim.x) {
+    unsigned turn = 0;
+    for (uint64_t i = blockIdx.x; i < todo; i += gridDim.x, turn ^= 1) {
+        Tx *const ptx = ptxs[turn];
         const uint64_t b = redo ? redo[1 + i] : i;
         const uint64_t first = b * SEQ_TILE + warp * SEQ_PIECE + lane;
         const int e = guess[b];
@@ -319,12 +359,20 @@ __global__ void __launch_bounds__(SEQ_TPB, 4) k_seq_steps(Prod pr, uint64_t coun
         using P = decltype(pr.p(uint64_t(0)));
         StepSum<A, P> mine(e);
         bool nonzero = false;
-#pragma unroll 8
-        for (int k = 0; k < SEQ_PIECE; k += 32) {
-            if (first + k < count) {
-                const P p = pr.p(first + k);
-                nonzero |= to_bits(p) != 0;
-                if (any) mine.add(p);
+#pragma unroll 1
+        for (int k = 0; k < SEQ_PIECE; k += 32 * SEQ_AHEAD) {
+            decltype(pr.amp(uint64_t(0))) a[SEQ_AHEAD];
+            P p[SEQ_AHEAD];
+#pragma unroll
+            for (int u = 0; u < SEQ_AHEAD; u++) {
+                a[u].x = a[u].y = P(0);
+                if (first + k + 32 * u < count) a[u] = pr.amp(first + k + 32 * u);
+            }
+            norms<false>(a, p);
+#pragma unroll
+            for (int u = 0; u < SEQ_AHEAD; u++) {
+                nonzero |= to_bits(p[u]) != 0;
+                if (any) mine.add(p[u]);
             }
         }
         bool big = mine.big;
@@ -344,15 +392,20 @@ __global__ void __launch_bounds__(SEQ_TPB, 4) k_seq_steps(Prod pr, uint64_t coun
                 t = tx_then(t, all);
             }
         }
+        const unsigned saw = (__any_sync(0xffffffffu, big) ? 1u : 0u) | (__any_sync(0xffffffffu, nonzero) ? 2u : 0u);
         if (lane == 0) {
             ptx[warp] = t;
+            seen[turn][warp] = saw;
             if (pieces) {
                 pieces[2 * (b * SEQ_PIECES + warp)] = t.d[0];
                 pieces[2 * (b * SEQ_PIECES + warp) + 1] = t.d[1];
             }
         }
-        const bool big_all = __syncthreads_or(big) != 0;
-        const bool some = __syncthreads_or(nonzero) != 0;
+        __syncthreads();
+        unsigned all = 0;
+#pragma unroll
+        for (int w = 0; w < SEQ_PIECES; w++) all |= seen[turn][w];
+        const bool big_all = (all & 1u) != 0, some = (all & 2u) != 0;
         const bool lost = big_all || (!any && some);
         if (lost) {                                       // the steps do not give the tile's sum
             double acc = 0;
@@ -378,7 +431,6 @@ __global__ void __launch_bounds__(SEQ_TPB, 4) k_seq_steps(Prod pr, uint64_t coun
             else if (some) sum_est = ldexp(double(tot.d[0]), e - fp_traits<A>::MANT);
             est[b] = sum_est;
         }
-        __syncthreads();
     }
 }
 
@@ -651,12 +703,15 @@ __global__ void __launch_bounds__(SEQ_WALK_TPB) k_seq_walk(Prod pr, uint64_t cou
             const uint64_t base = t * SEQ_TILE;
             const unsigned valid = unsigned(count - base < uint64_t(SEQ_TILE) ? count - base : uint64_t(SEQ_TILE));
             __syncthreads();
+            decltype(pr.amp(uint64_t(0))) a[SEQ_TERMS];
             P v[SEQ_TERMS];
 #pragma unroll
             for (int r = 0; r < SEQ_TERMS; r++) {
                 const unsigned i = unsigned(r) * SEQ_WALK_TPB + tid;
-                v[r] = i < valid ? pr.p(base + i) : P(0);
+                a[r].x = a[r].y = P(0);
+                if (i < valid) a[r] = pr.amp(base + i);
             }
+            norms<true>(a, v);
 #pragma unroll
             for (int r = 0; r < SEQ_TERMS; r++) tm[term_slot(unsigned(r) * SEQ_WALK_TPB + tid)] = v[r];
             __syncthreads();

@@ -44,3 +44,26 @@ def test_walked_sums_and_shots_match_oracle(qsl, port, n, dtype):
         for q, o in ((0, 0), (n - 1, 1), (n // 2, 0)):
             assert gpu.prob(q, o) == cpu.prob(q, o), (name, q, o)
         assert np.array_equal(gpu.sample_shots(u), cpu.sample_all(u)), name
+
+
+@pytest.mark.parametrize("n", [6, 13, 18])
+def test_terms_with_and_without_easy_squares(qsl, port, n):
+    # |a|^2 on the integer pipes takes parts with exponent fields 512 to 1533 and a low bit set; a warp
+    # with any other part takes the FP64 pipe.  Whole stretches of each kind, and single parts among easy ones.
+    rng = np.random.default_rng(n)
+    dim = 1 << n
+    st = rng.normal(size=dim) + 1j * rng.normal(size=dim)
+    st /= np.linalg.norm(st)
+    v = st.view(np.float64)
+    odd = np.array([0.0, -0.0, 2.0 ** -511, np.nextafter(2.0 ** -511, 0), 2.0 ** -512, 1e-200, 5e-324, 2.0 ** -5, 1.5 * 2.0 ** -9,
+                    1 + 2.0 ** -26, 2.0 ** -7 * (1 + 2.0 ** -25)])
+    odd[-2:] *= 2.0 ** -6
+    few = rng.random(v.size) < 0.02
+    v[few] = rng.choice(odd, few.sum())
+    v[v.size // 4: v.size // 4 + v.size // 8] = rng.choice(odd[:7], v.size // 8)
+    u = rng.random(200)
+    gpu, cpu = qsl.Qubits(n, state=st), port.PortQubits(n, state=st)
+    for q in range(0, n, 3):
+        for o in (0, 1):
+            assert gpu.prob(q, o) == cpu.prob(q, o), (q, o)
+    assert np.array_equal(gpu.sample_shots(u), cpu.sample_all(u))
