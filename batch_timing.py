@@ -11,8 +11,8 @@ one k_batch launch after a warm-up run (`-s 1 -c 1`):
     python batch_timing.py [--first 12] [--largest 4] [--dtype c128] [--repeat 3]
                            [--shape THREADS,TILE_LOG2,CTAS_PER_SM] [--max-qubits N]
 
-Without `--shape` the batch keeps its default launch shape (1024 threads,
-one CTA per SM, the larger tile); the benchmark's autotuner picks among
+Without `--shape` the batch keeps its default launch shape (complex128: 1024
+threads, complex64: 512; one CTA per SM, the larger tile); the benchmark's autotuner picks among
 the shapes `Batch.shapes()` lists.
 """
 from __future__ import annotations

@@ -531,6 +531,24 @@ def launch_windows(layer, grouping=True):
     return out
 
 
+def timed_windows(layer, grouping=True):
+    """launch_windows with the two-qubit gates that follow one another joined:
+    the library holds these too and chooses between one sweep each and runs of
+    several, so they are timed together, closed by a flush.  Returns
+    (calls, gates) pairs; a call of None is a flush."""
+    out = []
+    for call, gates in launch_windows(layer, grouping):
+        two = grouping and gates == [call] and call[2] is not None
+        if two and out and out[-1][2]:
+            calls, held, _ = out.pop()
+            out.append((calls[:-1] + [call, None], held + gates, True))
+        elif two:
+            out.append(([call, None], gates, True))
+        else:
+            out.append(([call], gates, False))
+    return [(calls, gates) for calls, gates, _ in out]
+
+
 def roofline_of(args, name, top, peak, peak_kind):
     """The roofline object of the dominant kernel: its algorithmic bytes per
     launch (the reference's count, 2 x 16 B x amplitudes changed, for every
@@ -583,7 +601,7 @@ def run_gpu(args):
 
     def timed(timing, fn, launched):
         """Run fn; with `timing`, inside a pair of events on the stream,
-        recorded with the gates of the kernel it launches (None: none)."""
+        recorded with the gates that it launches (None: none)."""
         if timing is None:
             fn()
             return
@@ -596,11 +614,14 @@ def run_gpu(args):
             timing.append((launched, e0, e1))
 
     def run_layer(li, timing):
-        for call, launched in launch_windows(layers[li % len(layers)], grouping):
-            if call is None:
-                timed(timing, sim.flush, launched)
-            else:
-                timed(timing, lambda: sim.gate(*call), launched)
+        for calls, launched in timed_windows(layers[li % len(layers)], grouping):
+            def run():
+                for call in calls:
+                    if call is None:
+                        sim.flush()
+                    else:
+                        sim.gate(*call)
+            timed(timing, run, launched)
 
     # warm-up layers (the circuit's own first layers)
     for w in range(args.warmup):
@@ -634,7 +655,8 @@ def run_gpu(args):
     per = {}
     for gs, e0, e1 in timing:
         ms = e0.elapsed_time(e1)
-        name = "k_group2" if len(gs) == 2 else kernel_of(gs[0][0])
+        two = grouping and gs[0][2] is not None
+        name = "two-qubit gates" if two else "k_group2" if len(gs) == 2 else kernel_of(gs[0][0])
         d = per.setdefault(name, {"launches": 0, "ms": 0.0, "bytes": 0, "gates": 0})
         d["launches"] += 1
         d["ms"] += ms

@@ -311,8 +311,8 @@ QSLC_API int qslc_batch_destroy(qslc_batch *b);
  * library in one process are serialised).  States above
  * QSLC_NOALLOC_MAX_QUBITS qubits (and nqubits == 0) are rejected with
  * QSLC_EINVAL before anything else is done.  Each call blocks until the
- * result is on the host: it synchronises `stream` and copies into fixed
- * host arrays, so it must not be called while that stream (or, in global
+ * result is on the host: it synchronises `stream` and copies the result,
+ * so it must not be called while that stream (or, in global
  * capture mode, any stream) is being captured.  The first call on a device
  * looks up the array's address on that device and keeps it for the life of
  * the process; do not use the library across a cudaDeviceReset. */
