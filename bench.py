@@ -84,7 +84,7 @@ def kernel_of(gate: str) -> str:
 # so next to the number, and --traffic replaces it with a capture's figure.
 K_PAIR1_TRAFFIC_RATIO = 2.086 / 2.147
 # The same for the grouped sweep of two rotations on a dense 26-qubit state:
-# 1.074 + 1.012 GB of DRAM traffic for the two gates' 2 x 2.147 GB.
+# 1.074 + 1.033 GB of DRAM traffic for the two gates' 2 x 2.147 GB.
 K_GROUP2_TRAFFIC_RATIO = (1.074 + 1.033) / (2 * 2.147)
 
 
