@@ -202,9 +202,9 @@ __device__ __forceinline__ void diag_update(cplx<T> &a, const Coef<T> &k, unsign
 // Updates of easy operands (lean.cuh): products and divisions on the integer
 // pipes, one FP64 add per output.  Each returns whether it ran; when it did
 // not, the amplitudes are unchanged and the caller takes the general update.
-// The test is a vote of the warp, so a warp with a zero (or otherwise not
-// easy) operand runs the general update alone and never both.  Only a
-// quotient that lean_div could not decide is left to its own thread.
+// Each thread decides for itself, with no vote: the updates are called from
+// divergent code (items past a sweep's end, controls tested per thread), where
+// no mask is known that names exactly the lanes of a vote.
 //
 // Bound by the FP64 pipe (two operations per SM and clock) and the ALU pipe
 // together: 98 instructions per amplitude and gate against 150 with the
@@ -212,8 +212,6 @@ __device__ __forceinline__ void diag_update(cplx<T> &a, const Coef<T> &k, unsign
 // 26-qubit dense state in one sweep: 757 us with the general split, 570 us
 // with this; FP64 pipe 72% busy, ALU pipe 58%.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool warp_all(bool x) { return __all_sync(__activemask(), x); }
-
 __device__ __forceinline__ double lean_prod(const emu::LeanOp &a, const emu::LeanK &k)
 {
     return emu::dfrom(emu::lean_mul(a, k));
@@ -226,11 +224,10 @@ __device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const Coef<d
         double s0 = __dadd_rn(a0.x, a1.x), s1 = __dadd_rn(a0.y, a1.y);
         double d0 = __dsub_rn(a0.x, a1.x), d1 = __dsub_rn(a0.y, a1.y);
         // opaque from here: the compiler would otherwise compute the sums a
-        // second time after the vote, and the FP64 pipe is what binds
+        // second time after the test, and the FP64 pipe is what binds
         asm volatile("" : "+d"(s0), "+d"(s1), "+d"(d0), "+d"(d1));
         const uint64_t b0 = emu::dbits(s0), b1 = emu::dbits(s1), b2 = emu::dbits(d0), b3 = emu::dbits(d1);
-        if (!warp_all(k.ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) &
-                                         emu::easy_range(b3)))
+        if (!(k.ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) & emu::easy_range(b3)))
             return false;
         bool sure = true;
         const uint64_t q0 = emu::lean_div(emu::lean_operand(b0), k.ld, sure);
@@ -243,8 +240,8 @@ __device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const Coef<d
         return true;
     } else {
         const uint64_t b0 = emu::dbits(a0.x), b1 = emu::dbits(a0.y), b2 = emu::dbits(a1.x), b3 = emu::dbits(a1.y);
-        if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(b0) & emu::easy_product(b1) &
-                                                              emu::easy_product(b2) & emu::easy_product(b3)))
+        if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(b0) & emu::easy_product(b1) &
+                                                      emu::easy_product(b2) & emu::easy_product(b3)))
             return false;
         const emu::LeanOp x0 = emu::lean_operand(b0), y0 = emu::lean_operand(b1);
         const emu::LeanOp x1 = emu::lean_operand(b2), y1 = emu::lean_operand(b3);
@@ -273,7 +270,7 @@ template <int OP>
 __device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
 {
     const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y);
-    if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
+    if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
     const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
     const double xc = lean_prod(x, k.lc), ys = lean_prod(y, k.ls), yc = lean_prod(y, k.lc), xs = lean_prod(x, k.ls);
     a.x = OP == D_PHASE ? __dsub_rn(xc, ys) : __dadd_rn(xc, ys);
@@ -285,7 +282,7 @@ __device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
 __device__ __forceinline__ bool phase_flip_lean(double2 &a, uint32_t flip, const Coef<double> &k)
 {
     const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y), f = uint64_t(flip) << 32;
-    if (!warp_all((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
+    if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
     const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
     const double xc = lean_prod(x, k.lc), ys = emu::dfrom(emu::lean_mul(y, k.ls) ^ f);
     const double yc = lean_prod(y, k.lc), xs = emu::dfrom(emu::lean_mul(x, k.ls) ^ f);
@@ -360,7 +357,7 @@ constexpr int ITEMS = QSLC_ITEMS;
 constexpr unsigned PAT_RUNTIME = 0xFFFFFFFFu;
 
 // PAT_LEAN, the default of the complex128 sweeps: the easy form first
-// (pair_gate, diag_gate), with the default pattern for the warps it leaves.
+// (pair_gate, diag_gate), with the default pattern for the operands it leaves.
 constexpr unsigned PAT_LEAN = 0xFFFFFFFEu;
 
 // The default splits of the general path.  A pattern holds one 8-bit mode
@@ -371,8 +368,8 @@ constexpr unsigned PAT_ROT = 0x959595u;
 constexpr unsigned PAT_H = 0u;
 constexpr unsigned PAT_DIAG = 0x090909u;
 
-// The general update of the warps that the easy forms leave.  A warp whose operands are all +0 (most of a sparse
-// state) only needs the signs of its zeros, which follow from the signs of
+// The general update of the operands that the easy forms leave.  Operands that are all +0 (most of a sparse
+// state) only need the signs of their zeros, which follow from the signs of
 // the coefficients: a sum of two zeros is -0 when both are, a difference p - q
 // when p is -0 and q is +0.
 //
@@ -416,7 +413,7 @@ template <int OP>
 __device__ __forceinline__ Pair pair_general(double2 a0, double2 a1, const SlowCoef *q)
 {
     const Coef<double> k = general_coef(q);
-    if (warp_all(plus_zero(a0) & plus_zero(a1))) {
+    if (plus_zero(a0) & plus_zero(a1)) {
         const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
         const double add = zero_of(c & s), sub = zero_of(c & ~s);
         if constexpr (OP == P_RX) a0 = a1 = make_double2(add, sub);
@@ -438,7 +435,7 @@ __device__ __forceinline__ Pair hadamard_general(double2 a0, double2 a1, double 
     k.c = r;
     k.kd = *kd;
     // +0 +- +0 is +0, and so is its quotient
-    if (!warp_all(plus_zero(a0) & plus_zero(a1))) pair_update<double, P_H>(a0, a1, k, PAT_H & 0xFFu);
+    if (!(plus_zero(a0) & plus_zero(a1))) pair_update<double, P_H>(a0, a1, k, PAT_H & 0xFFu);
     return Pair{a0, a1};
 }
 // x c - y s, y c + x s (INV: s with its sign flipped)
@@ -447,7 +444,7 @@ __device__ __forceinline__ double2 phase_general(double2 a, const SlowCoef *q)
 {
     const Coef<double> k = general_coef(q);
     const double x = a.x, y = a.y;
-    if (warp_all(plus_zero(a))) {
+    if (plus_zero(a)) {
         const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
         const double add = zero_of(c & s), sub = zero_of(c & ~s);
         return INV ? make_double2(add, sub) : make_double2(sub, add);

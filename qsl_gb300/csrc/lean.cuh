@@ -5,8 +5,8 @@
 // for its range, and shifts every product into place after multiplying.
 // The forms here take only "easy" operands -- normal, exponent field 65 to
 // 2044, low significand word not zero -- and leave every other operand to
-// the caller, which tests them first (easy_bits) and sends the whole warp
-// through the general path when a lane has one that is not easy.  What the
+// the caller, which tests them first (easy_range, easy_product) and sends a
+// thread through the general path when it has one that is not easy.  What the
 // restriction buys:
 //   - no zero handling, and no rounding ties: a product lies half-way
 //     between two doubles only when the operand's significand has at least
