@@ -371,7 +371,8 @@ constexpr unsigned PAT_DIAG = 0x090909u;
 // The general update of the operands that the easy forms leave.  Operands that are all +0 (most of a sparse
 // state) only need the signs of their zeros, which follow from the signs of
 // the coefficients: a sum of two zeros is -0 when both are, a difference p - q
-// when p is -0 and q is +0.
+// when p is -0 and q is +0.  That holds for finite coefficients: those of an
+// infinite or NaN angle are NaN, and so is their product with a zero.
 //
 // The sweeps of several gates call it out of line (pair_slow and the like):
 // inline, once per gate type and pair, it would double their code.  There the
@@ -405,6 +406,11 @@ __device__ __forceinline__ bool plus_zero(const double2 &a)
 {
     return (emu::dbits(a.x) | emu::dbits(a.y)) == 0;
 }
+// Whether c and s are finite; the sine and cosine of one angle are finite together.
+__device__ __forceinline__ bool finite_coef(const Coef<double> &k)
+{
+    return (__double2hiint(k.c) & 0x7FF00000) != 0x7FF00000;
+}
 
 struct Pair {
     double2 a0, a1;
@@ -413,7 +419,7 @@ template <int OP>
 __device__ __forceinline__ Pair pair_general(double2 a0, double2 a1, const SlowCoef *q)
 {
     const Coef<double> k = general_coef(q);
-    if (plus_zero(a0) & plus_zero(a1)) {
+    if (plus_zero(a0) & plus_zero(a1) & finite_coef(k)) {
         const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
         const double add = zero_of(c & s), sub = zero_of(c & ~s);
         if constexpr (OP == P_RX) a0 = a1 = make_double2(add, sub);
@@ -444,7 +450,7 @@ __device__ __forceinline__ double2 phase_general(double2 a, const SlowCoef *q)
 {
     const Coef<double> k = general_coef(q);
     const double x = a.x, y = a.y;
-    if (plus_zero(a)) {
+    if (plus_zero(a) & finite_coef(k)) {
         const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
         const double add = zero_of(c & s), sub = zero_of(c & ~s);
         return INV ? make_double2(add, sub) : make_double2(sub, add);
