@@ -99,7 +99,9 @@ QSLC_API int qslc_create_np(unsigned nqubits, unsigned nones, int dtype, qslc_st
 /* ~Qubits */
 QSLC_API int qslc_destroy(qslc_state *s);
 
-/* Qubits(const Qubits&) (default.hpp:137): a deep device-to-device copy. */
+/* Qubits(const Qubits&) (default.hpp:137): a deep device-to-device copy, on
+ * the new handle's stream.  What the source's stream is given after this call
+ * (and after qslc_assign) runs once the copy has read it. */
 QSLC_API int qslc_clone(const qslc_state *src, qslc_state **out);
 
 /* operator=(const Qubits&) (default.cpp:94-105): copies the amplitudes;

@@ -174,6 +174,24 @@ int check_handle(const qslc_state *s)
     return QSLC_OK;
 }
 
+// What is queued on `later` from here on runs after what is queued on
+// `earlier` so far.
+int order_after(cudaStream_t later, cudaStream_t earlier)
+{
+    if (later == earlier) return QSLC_OK;
+    cudaEvent_t ev = nullptr;
+    cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) {
+        e = cudaEventRecord(ev, earlier);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(later, ev, 0);
+        cudaEventDestroy(ev);                // released once the wait is over
+    }
+    if (e == cudaSuccess) return QSLC_OK;
+    cudaGetLastError();
+    QSLC_CUDA(cudaStreamSynchronize(earlier));
+    return QSLC_OK;
+}
+
 // Apply held and queued gates (the run held back; the precision form's queue) before the state is read, and report a staged sweep whose
 // barrier wait ran out since the last check.
 int flushed(qslc_state *s)
@@ -388,6 +406,7 @@ int qslc_clone(const qslc_state *src, qslc_state **out)
         cudaError_t e = cudaMemcpyAsync(s->amps, src->amps, src->namps * src->amp_bytes(),
                                         cudaMemcpyDeviceToDevice, s->stream);
         if (e != cudaSuccess) rc = cuda_fail(e, "clone copy");
+        else rc = order_after(src->stream, s->stream);   // the source stays as it is until it is copied
     }
     if (rc) {
         free_state(s);
@@ -426,7 +445,7 @@ int qslc_assign(qslc_state *dst, const qslc_state *src)
     QSLC_CUDA(cudaStreamSynchronize(src->stream));
     QSLC_CUDA(cudaMemcpyAsync(dst->amps, src->amps, src->namps * src->amp_bytes(),
                               cudaMemcpyDeviceToDevice, dst->stream));
-    return QSLC_OK;
+    return order_after(src->stream, dst->stream);        // the source stays as it is until it is copied
 }
 
 unsigned qslc_num_qubits(const qslc_state *s) { return s ? s->n : 0; }
