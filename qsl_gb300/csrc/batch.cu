@@ -1006,8 +1006,9 @@ int capture(qslc_batch *b, const BatchShape &s)
         }
         b->arena_bytes = need;
     }
+    // after the last run, which reads it, and before the next
+    QSLC_CUDA(cudaMemcpyAsync(b->d_order, order.data(), b->ninst * 4, cudaMemcpyHostToDevice, b->stream));
     QSLC_CUDA(cudaStreamSynchronize(b->stream));
-    QSLC_CUDA(cudaMemcpy(b->d_order, order.data(), b->ninst * 4, cudaMemcpyHostToDevice));
     BatchArgs a;
     a.inst = static_cast<const InstDesc *>(b->d_inst);
     a.order = static_cast<const uint32_t *>(b->d_order);
@@ -1229,14 +1230,16 @@ extern "C" int qslc_batch_create(int dtype, uint32_t ninst, const uint32_t *nqub
     alloc(&b->d_pick, size_t(sm_count()) * 8 * sizeof(unsigned));
     if (!rc && cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
         rc = fail(QSLC_ECUDA, "stream creation failed");
-    if (!rc && cudaMemcpy(b->d_inst, b->inst.data(), ninst * sizeof(InstDesc), cudaMemcpyHostToDevice) != cudaSuccess)
+    // on the batch's own stream, which does not wait for the default one
+    if (!rc && (cudaMemcpyAsync(b->d_inst, b->inst.data(), ninst * sizeof(InstDesc), cudaMemcpyHostToDevice,
+                                b->stream) != cudaSuccess ||
+                cudaMemcpyAsync(b->d_size_order, b->size_order.data(), ninst * 4, cudaMemcpyHostToDevice,
+                                b->stream) != cudaSuccess))
         rc = fail(QSLC_ECUDA, "upload failed");
     if (!rc && (cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
                 cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming) != cudaSuccess ||
                 cudaEventCreateWithFlags(&b->joined, cudaEventDisableTiming) != cudaSuccess))
         rc = fail(QSLC_ECUDA, "stream creation failed");
-    if (!rc && cudaMemcpy(b->d_size_order, b->size_order.data(), ninst * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-        rc = fail(QSLC_ECUDA, "upload failed");
     if (!rc) {
         const auto c = candidates(b);
         if (c.empty()) rc = fail(QSLC_EINVAL, "no launch shape fits the largest instance");

@@ -312,6 +312,9 @@ int init_once()
             }
     QSLC_CUDA(cudaMalloc(&d_rank_tab, rt.size() * 4));
     QSLC_CUDA(cudaMemcpy(d_rank_tab, rt.data(), rt.size() * 4, cudaMemcpyHostToDevice));
+    // both calls may return with the data staged only, and the handles' streams
+    // do not wait for the default one
+    QSLC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     return QSLC_OK;
 }
 
