@@ -597,7 +597,10 @@ def run_gpu(args):
     sim = q.Qubits(n)
     sim.set_stream(stream.cuda_stream)
 
-    grouping = os.environ.get("QSLC_GROUP", "1")[:1] != "0"
+    # the library holds no gates with QSLC_GROUP=0, nor with a switch of the single sweeps
+    sweeps = ("QSLC_EMU_MASK", "QSLC_EMU_MASK_H", "QSLC_EMU_MASK_DIAG", "QSLC_BULK", "QSLC_SHFL")
+    group = os.environ.get("QSLC_GROUP") or ("0" if any(os.environ.get(v) for v in sweeps) else "1")
+    grouping = group[:1] != "0"
 
     def timed(timing, fn, launched):
         """Run fn; with `timing`, inside a pair of events on the stream,

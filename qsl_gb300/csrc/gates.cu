@@ -840,11 +840,15 @@ int group2_t(qslc_state *s, const GateOp &g0, const GateOp &g1)
 
 }  // namespace
 
+// The switches that choose the form of a gate's own sweep mean that sweep:
+// with one of them set, gates are not held unless QSLC_GROUP says so.
 GroupMode group_mode()
 {
     static const GroupMode m = [] {
-        const char *e = std::getenv("QSLC_GROUP");
-        return !e || !*e ? GROUP_RUNS : e[0] == '0' ? GROUP_OFF : GROUP_PAIRS;
+        if (!unset("QSLC_GROUP")) return std::getenv("QSLC_GROUP")[0] == '0' ? GROUP_OFF : GROUP_PAIRS;
+        for (const char *v : {"QSLC_EMU_MASK", "QSLC_EMU_MASK_H", "QSLC_EMU_MASK_DIAG", "QSLC_BULK", "QSLC_SHFL"})
+            if (!unset(v)) return GROUP_OFF;
+        return GROUP_RUNS;
     }();
     return m;
 }

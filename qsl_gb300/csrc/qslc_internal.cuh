@@ -178,7 +178,8 @@ int launch_gate2(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle
 // two one-qubit gates on different qubits, in this order, in one sweep
 int launch_group2(qslc_state *s, const GateOp &g0, const GateOp &g1);
 // How gates on a plain state are held back (QSLC_GROUP): not at all ("0"),
-// one-qubit gates two to a sweep ("1"), or runs of any gates (unset).
+// one-qubit gates two to a sweep ("1"), or runs of any gates (unset, with
+// the switches of single sweeps unset too).
 enum GroupMode { GROUP_OFF, GROUP_PAIRS, GROUP_RUNS };
 GroupMode group_mode();
 // Debug builds (-DQSLC_DEBUG_BOUNDS): QSLC_EINVAL when a sweep met an index
