@@ -19,6 +19,7 @@
 // sum, and so does every update below (rn<T>::mul/add/sub/div, and for
 // complex128 the integer forms of the same operations, gatemath.cuh).
 #include "qslc_internal.cuh"
+#include "bounds.cuh"
 #include "gatemath.cuh"
 #include "gateops.cuh"
 #include "stage.cuh"
@@ -30,29 +31,6 @@
 
 namespace qslc {
 namespace {
-
-// Debug builds (-DQSLC_DEBUG_BOUNDS) check each item's largest index
-// against the state's size before the item is read or written: an index
-// outside the state is recorded (the first one) and the item skipped, and
-// the next call that reads the state returns QSLC_EINVAL with the index
-// (debug_bounds_error).  The host validates every qubit index before a
-// launch, so no call through the ABI should record one.  Default builds
-// compile both checks to `true`.
-#ifdef QSLC_DEBUG_BOUNDS
-__device__ unsigned long long g_bad_index;   // first index outside a state, plus one; 0: none
-__device__ __forceinline__ bool in_state(uint64_t i, uint64_t dim)
-{
-    if (i < dim) return true;
-    atomicCAS(&g_bad_index, 0ull, (unsigned long long)i + 1ull);
-    return false;
-}
-#define QSLC_IN_STATE(i, dim) in_state(uint64_t(i), uint64_t(dim))
-#define QSLC_IN_STATE_QUIET(i, dim) (uint64_t(i) < uint64_t(dim))
-#else
-#define QSLC_IN_STATE(i, dim) true
-#define QSLC_IN_STATE_QUIET(i, dim) true
-#endif
-
 
 // One-qubit pair gates: pairs (i0, i0 + 2^t), i0 = insert0(j, t).
 template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
@@ -860,18 +838,8 @@ int launch_group2(qslc_state *s, const GateOp &g0, const GateOp &g1)
 
 int debug_bounds_error()
 {
-#ifdef QSLC_DEBUG_BOUNDS
-    unsigned long long bad = 0;
-    QSLC_CUDA(cudaDeviceSynchronize());
-    QSLC_CUDA(cudaMemcpyFromSymbol(&bad, g_bad_index, sizeof(bad)));
-    if (bad) {
-        const unsigned long long zero = 0;
-        QSLC_CUDA(cudaMemcpyToSymbol(g_bad_index, &zero, sizeof(zero)));
-        return fail(QSLC_EINVAL, "a sweep indexed outside the state (debug bounds check): index " +
-                                     std::to_string(bad - 1));
-    }
-#endif
-    return QSLC_OK;
+    const int rc = unit_bounds_error(), run = run_bounds_error();
+    return rc ? rc : run;
 }
 
 int launch_gate1(qslc_state *s, int gate, unsigned targ, double angle)

@@ -186,6 +186,7 @@ GroupMode group_mode();
 // outside its state since the last call; QSLC_OK otherwise and in default
 // builds.
 int debug_bounds_error();
+int run_bounds_error();          // run.cu's part of it
 int launch_collapse(qslc_state *s, unsigned targ, unsigned outcome, double factor);
 // complex64 collapse with the factor applied in double (precision form)
 int launch_collapse_f64(qslc_state *s, unsigned targ, unsigned outcome, double factor);

@@ -21,6 +21,7 @@
 // the traffic (four such layers: 5.6 ms before, 2.7 ms).  complex128 runs
 // are bound by the FP64 and ALU pipes as the single sweeps are, and gain where
 // launches or moves count: 8 layers of 10 qubits 418 -> 203 us.
+#include "bounds.cuh"
 #include "gatemath.cuh"
 
 #include <algorithm>
@@ -282,10 +283,12 @@ __global__ void __launch_bounds__(256, RUN_CTAS)
             cplx<T> v[RUN_LOADS];
 #pragma unroll
             for (int u = 0; u < RUN_LOADS; u++)
-                if (i0 + u < rounds) v[u] = mem[a.chunk[i0 + u]];
+                if (i0 + u < rounds && QSLC_IN_STATE((tile | mine) + a.chunk[i0 + u], a.ntiles << a.bits))
+                    v[u] = mem[a.chunk[i0 + u]];
 #pragma unroll
             for (int u = 0; u < RUN_LOADS; u++)
-                if (i0 + u < rounds) at(home ^ (slot_of<T>((i0 + u) * nt) * AB)) = v[u];
+                if (i0 + u < rounds && QSLC_IN_STATE_QUIET((tile | mine) + a.chunk[i0 + u], a.ntiles << a.bits))
+                    at(home ^ (slot_of<T>((i0 + u) * nt) * AB)) = v[u];
         }
         __syncthreads();
         for (int s = 0; s < a.nsteps; s++) {
@@ -327,7 +330,8 @@ __global__ void __launch_bounds__(256, RUN_CTAS)
         for (int i0 = 0; i0 < rounds; i0 += RUN_LOADS) {
 #pragma unroll
             for (int u = 0; u < RUN_LOADS; u++)
-                if (i0 + u < rounds) mem[a.chunk[i0 + u]] = at(home ^ (slot_of<T>((i0 + u) * nt) * AB));
+                if (i0 + u < rounds && QSLC_IN_STATE_QUIET((tile | mine) + a.chunk[i0 + u], a.ntiles << a.bits))
+                    mem[a.chunk[i0 + u]] = at(home ^ (slot_of<T>((i0 + u) * nt) * AB));
         }
     }
 }
@@ -717,6 +721,8 @@ int run_push(qslc_state *s, const GateOp &g)
     if (mode == GROUP_OFF || (pairs && (is_two_qubit(g.code) || s->run.size() == 2))) return run_release(s);
     return QSLC_OK;
 }
+
+int run_bounds_error() { return unit_bounds_error(); }
 
 void run_drop(qslc_state *s)
 {
