@@ -108,7 +108,8 @@ struct LayerCoefs {
 __device__ __forceinline__ BatchCoef<float> batch_coef(float c, float s) { return BatchCoef<float>{c, s}; }
 __device__ __forceinline__ BatchCoef<double> batch_coef(double c, double s)
 {
-    return BatchCoef<double>{emu::make_lean(c), emu::make_lean(s), SlowCoef{c, s, emu::make_mulk(c), emu::make_mulk(s)}};
+    return BatchCoef<double>{emu::make_lean_gate(c), emu::make_lean_gate(s),
+                             SlowCoef{c, s, emu::make_mulk(c), emu::make_mulk(s)}};
 }
 
 template <class T>
@@ -187,7 +188,7 @@ __device__ __forceinline__ void rz_regs(double2 (&v)[4], const BatchCoef<double>
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const uint32_t flip = ((ones >> i) & 1u) ? 0u : 0x80000000u;
-        if (!phase_flip_lean(v[i], flip, k)) v[i] = flip ? phase_slow<true>(v[i], &bc.head) : phase_slow<false>(v[i], &bc.head);
+        phase_flip(v[i], flip, k, &bc.head);
     }
 }
 __device__ __forceinline__ void rz_regs(float2 (&v)[1 << BR<float>], const BatchCoef<float> &bc, unsigned ones)

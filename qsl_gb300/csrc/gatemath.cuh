@@ -207,87 +207,157 @@ __device__ __forceinline__ void diag_update(cplx<T> &a, const Coef<T> &k, unsign
 // no mask is known that names exactly the lanes of a vote.
 //
 // Bound by the FP64 pipe (two operations per SM and clock) and the ALU pipe
-// together: 98 instructions per amplitude and gate against 150 with the
+// together: 96 instructions per amplitude and gate against 150 with the
 // general split "PPPQ", 2 of them FP64 instead of 2.7.  Two rotateX gates of a
-// 26-qubit dense state in one sweep: 757 us with the general split, 570 us
-// with this; FP64 pipe 72% busy, ALU pipe 58%.
+// 26-qubit dense state in one sweep: 761 us with the general split, 550 us
+// with this; FP64 pipe 79% busy.
+//
+// Three forms, from the cheapest: easy operands; operands that are easy or
+// zero; any.  Constants may be powers of two (make_lean_gate), so quarter turns
+// are easy too: two rotateX(pi) 885 us without, 550 with.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double lean_prod(const emu::LeanOp &a, const emu::LeanK &k)
+// Every rotation and phase is made of turns of two parts (u, v) to
+// (u c - v s, v c + u s), with s negated for INV: rotateX turns (a0.x, a1.y) and
+// (a1.x, a0.y), rotateY (a0.x, a1.x) and (a0.y, a1.y), rotateZ and phase the
+// parts of one amplitude.  `flip` (0x80000000 or 0) negates s at run time.
+template <class Op>
+__device__ __forceinline__ double lean_prod(const Op &a, const emu::LeanK &k, uint32_t flip = 0)
 {
-    return emu::dfrom(emu::lean_mul(a, k));
+    return emu::dfrom(emu::lean_mul(a, k) ^ (uint64_t(flip) << 32));
+}
+template <bool INV, class Op>
+__device__ __forceinline__ void turn(double &u, double &v, const Op &a, const Op &b, const emu::LeanK &lc,
+                                     const emu::LeanK &ls, uint32_t flip)
+{
+    const double uc = lean_prod(a, lc), vs = lean_prod(b, ls, flip), vc = lean_prod(b, lc), us = lean_prod(a, ls, flip);
+    u = INV ? __dadd_rn(uc, vs) : __dsub_rn(uc, vs);
+    v = INV ? __dsub_rn(vc, us) : __dadd_rn(vc, us);
+}
+template <bool INV>
+__device__ __forceinline__ void turn_easy(double &u, double &v, const emu::LeanK &lc, const emu::LeanK &ls,
+                                          uint32_t flip = 0)
+{
+    turn<INV>(u, v, emu::lean_operand(emu::dbits(u)), emu::lean_operand(emu::dbits(v)), lc, ls, flip);
+}
+__device__ __forceinline__ double zero_of(uint32_t sign)
+{
+    return __hiloint2double(int(sign & 0x80000000u), 0);
+}
+// The turn of two zeros: a sum of two zeros is -0 when both are, a difference
+// p - q when p is -0 and q is +0.  csign, ssign: the signs of c and s.
+template <bool INV>
+__device__ __forceinline__ void turn_signs(double &u, double &v, uint32_t csign, uint32_t ssign)
+{
+    const uint32_t a = uint32_t(__double2hiint(u)), b = uint32_t(__double2hiint(v)), t = INV ? ssign : ~ssign;
+    u = zero_of((a ^ csign) & (b ^ t));
+    v = zero_of((b ^ csign) & (a ^ ~t));
+}
+// The turn of parts that are easy or zeros: the zeros of a real state's imaginary
+// parts, say, only take signs.
+template <bool INV>
+__device__ __forceinline__ void turn_zeros(double &u, double &v, const emu::LeanK &lc, const emu::LeanK &ls,
+                                           uint32_t flip = 0)
+{
+    const uint64_t a = emu::dbits(u), b = emu::dbits(v);
+    if (emu::is_zero(a) & emu::is_zero(b)) turn_signs<INV>(u, v, emu::lean_sign(lc), emu::lean_sign(ls) ^ flip);
+    else turn<INV>(u, v, emu::lean_operand_z(a), emu::lean_operand_z(b), lc, ls, flip);
 }
 
-template <int OP>
-__device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const Coef<double> &k)
+template <int OP, class F, class G>
+__device__ __forceinline__ void pair_turns(double2 &a0, double2 &a1, F &&turn_inv, G &&turn_fwd)
 {
-    if constexpr (OP == P_H) {
-        double s0 = __dadd_rn(a0.x, a1.x), s1 = __dadd_rn(a0.y, a1.y);
-        double d0 = __dsub_rn(a0.x, a1.x), d1 = __dsub_rn(a0.y, a1.y);
-        // opaque from here: the compiler would otherwise compute the sums a
-        // second time after the test, and the FP64 pipe is what binds
-        asm volatile("" : "+d"(s0), "+d"(s1), "+d"(d0), "+d"(d1));
-        const uint64_t b0 = emu::dbits(s0), b1 = emu::dbits(s1), b2 = emu::dbits(d0), b3 = emu::dbits(d1);
-        if (!(k.ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) & emu::easy_range(b3)))
-            return false;
-        bool sure = true;
-        const uint64_t q0 = emu::lean_div(emu::lean_operand(b0), k.ld, sure);
-        const uint64_t q1 = emu::lean_div(emu::lean_operand(b1), k.ld, sure);
-        const uint64_t q2 = emu::lean_div(emu::lean_operand(b2), k.ld, sure);
-        const uint64_t q3 = emu::lean_div(emu::lean_operand(b3), k.ld, sure);
-        if (!sure) return false;
-        a0 = make_double2(emu::dfrom(q0), emu::dfrom(q1));
-        a1 = make_double2(emu::dfrom(q2), emu::dfrom(q3));
-        return true;
+    if constexpr (OP == P_RX) {
+        turn_inv(a0.x, a1.y);
+        turn_inv(a1.x, a0.y);
+    } else if constexpr (OP == P_RY) {
+        turn_fwd(a0.x, a1.x);
+        turn_fwd(a0.y, a1.y);
     } else {
-        const uint64_t b0 = emu::dbits(a0.x), b1 = emu::dbits(a0.y), b2 = emu::dbits(a1.x), b3 = emu::dbits(a1.y);
-        if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(b0) & emu::easy_product(b1) &
-                                                      emu::easy_product(b2) & emu::easy_product(b3)))
-            return false;
-        const emu::LeanOp x0 = emu::lean_operand(b0), y0 = emu::lean_operand(b1);
-        const emu::LeanOp x1 = emu::lean_operand(b2), y1 = emu::lean_operand(b3);
-        // the outputs' terms in pair_update's order
-        if constexpr (OP == P_RX) {
-            a0.x = __dadd_rn(lean_prod(x0, k.lc), lean_prod(y1, k.ls));
-            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(x1, k.ls));
-            a1.x = __dadd_rn(lean_prod(x1, k.lc), lean_prod(y0, k.ls));
-            a1.y = __dsub_rn(lean_prod(y1, k.lc), lean_prod(x0, k.ls));
-        } else if constexpr (OP == P_RY) {
-            a0.x = __dsub_rn(lean_prod(x0, k.lc), lean_prod(x1, k.ls));
-            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(y1, k.ls));
-            a1.x = __dadd_rn(lean_prod(x0, k.ls), lean_prod(x1, k.lc));
-            a1.y = __dadd_rn(lean_prod(y0, k.ls), lean_prod(y1, k.lc));
-        } else {
-            a0.x = __dadd_rn(lean_prod(x0, k.lc), lean_prod(y0, k.ls));
-            a0.y = __dsub_rn(lean_prod(y0, k.lc), lean_prod(x0, k.ls));
-            a1.x = __dsub_rn(lean_prod(x1, k.lc), lean_prod(y1, k.ls));
-            a1.y = __dadd_rn(lean_prod(y1, k.lc), lean_prod(x1, k.ls));
-        }
-        return true;
+        turn_inv(a0.x, a0.y);
+        turn_fwd(a1.x, a1.y);
     }
 }
 
-template <int OP>
-__device__ __forceinline__ bool phase_lean(double2 &a, const Coef<double> &k)
+__device__ __forceinline__ bool takes(double v) { return emu::easy_product(emu::dbits(v)); }
+__device__ __forceinline__ bool takes_zero(double v) { return takes(v) | emu::is_zero(emu::dbits(v)); }
+__device__ __forceinline__ bool zeros(const double2 &a)
 {
-    const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y);
-    if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
-    const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
-    const double xc = lean_prod(x, k.lc), ys = lean_prod(y, k.ls), yc = lean_prod(y, k.lc), xs = lean_prod(x, k.ls);
-    a.x = OP == D_PHASE ? __dsub_rn(xc, ys) : __dadd_rn(xc, ys);
-    a.y = OP == D_PHASE ? __dadd_rn(yc, xs) : __dsub_rn(yc, xs);
+    return emu::is_zero(emu::dbits(a.x)) & emu::is_zero(emu::dbits(a.y));
+}
+__device__ __forceinline__ bool takes(const double2 &a) { return takes(a.x) & takes(a.y); }
+__device__ __forceinline__ bool takes_zero(const double2 &a) { return takes_zero(a.x) & takes_zero(a.y); }
+
+template <int OP>
+__device__ __forceinline__ bool pair_lean(double2 &a0, double2 &a1, const emu::LeanK &lc, const emu::LeanK &ls)
+{
+    if (!((lc.usable & ls.usable) != 0 && takes(a0) & takes(a1))) return false;
+    pair_turns<OP>(a0, a1, [&](double &u, double &v) { turn_easy<true>(u, v, lc, ls); },
+                   [&](double &u, double &v) { turn_easy<false>(u, v, lc, ls); });
+    return true;
+}
+template <int OP>
+__device__ __forceinline__ bool pair_zeros(double2 &a0, double2 &a1, const emu::LeanK &lc, const emu::LeanK &ls)
+{
+    if (!((lc.usable & ls.usable) != 0 && takes_zero(a0) & takes_zero(a1))) return false;
+    pair_turns<OP>(a0, a1, [&](double &u, double &v) { turn_zeros<true>(u, v, lc, ls); },
+                   [&](double &u, double &v) { turn_zeros<false>(u, v, lc, ls); });
+    return true;
+}
+template <bool INV>
+__device__ __forceinline__ bool phase_lean(double2 &a, const emu::LeanK &lc, const emu::LeanK &ls, uint32_t flip = 0)
+{
+    if (!((lc.usable & ls.usable) != 0 && takes(a))) return false;
+    turn_easy<INV>(a.x, a.y, lc, ls, flip);
+    return true;
+}
+template <bool INV>
+__device__ __forceinline__ bool phase_zeros(double2 &a, const emu::LeanK &lc, const emu::LeanK &ls, uint32_t flip = 0)
+{
+    if (!((lc.usable & ls.usable) != 0 && takes_zero(a))) return false;
+    turn_zeros<INV>(a.x, a.y, lc, ls, flip);
     return true;
 }
 
-// x c - y s, y c + x s with s negated when `flip` is 0x80000000 (0 otherwise).
-__device__ __forceinline__ bool phase_flip_lean(double2 &a, uint32_t flip, const Coef<double> &k)
+// Hadamard's quotients of the sums s and differences d by sqrt(2).
+__device__ __forceinline__ bool quotients_lean(double2 &s, double2 &d, const emu::LeanDiv &ld)
 {
-    const uint64_t bx = emu::dbits(a.x), by = emu::dbits(a.y), f = uint64_t(flip) << 32;
-    if (!((k.lc.usable & k.ls.usable) != 0 && emu::easy_product(bx) & emu::easy_product(by))) return false;
-    const emu::LeanOp x = emu::lean_operand(bx), y = emu::lean_operand(by);
-    const double xc = lean_prod(x, k.lc), ys = emu::dfrom(emu::lean_mul(y, k.ls) ^ f);
-    const double yc = lean_prod(y, k.lc), xs = emu::dfrom(emu::lean_mul(x, k.ls) ^ f);
-    a.x = __dsub_rn(xc, ys);
-    a.y = __dadd_rn(yc, xs);
+    const uint64_t b0 = emu::dbits(s.x), b1 = emu::dbits(s.y), b2 = emu::dbits(d.x), b3 = emu::dbits(d.y);
+    if (!(ld.usable && emu::easy_range(b0) & emu::easy_range(b1) & emu::easy_range(b2) & emu::easy_range(b3)))
+        return false;
+    bool sure = true;
+    const uint64_t q0 = emu::lean_div(emu::lean_operand(b0), ld, sure);
+    const uint64_t q1 = emu::lean_div(emu::lean_operand(b1), ld, sure);
+    const uint64_t q2 = emu::lean_div(emu::lean_operand(b2), ld, sure);
+    const uint64_t q3 = emu::lean_div(emu::lean_operand(b3), ld, sure);
+    if (!sure) return false;
+    s = make_double2(emu::dfrom(q0), emu::dfrom(q1));
+    d = make_double2(emu::dfrom(q2), emu::dfrom(q3));
+    return true;
+}
+// The same with zeros, their own quotients: a part whose sum and difference are zeros
+// (a real state's imaginary one) is left as it is.  False, with the values
+// unchanged, when one needs the general division.
+__device__ __forceinline__ bool quotients_zeros(double2 &s, double2 &d, const emu::LeanDiv &ld)
+{
+    bool sure = ld.usable != 0;
+    double2 qs = s, qd = d;
+    auto part = [&](double &x, double &y) {
+        const uint64_t a = emu::dbits(x), b = emu::dbits(y);
+        const bool za = emu::is_zero(a), zb = emu::is_zero(b);
+        if (za & zb) return;
+        sure = sure & (za | emu::easy_range(a)) & (zb | emu::easy_range(b));
+        bool sa = true, sb = true;
+        const double u = emu::dfrom(emu::lean_div(emu::lean_operand(a), ld, sa));
+        const double v = emu::dfrom(emu::lean_div(emu::lean_operand(b), ld, sb));
+        sure = sure & (za | sa) & (zb | sb);
+        x = za ? x : u;
+        y = zb ? y : v;
+    };
+    part(qs.x, qd.x);
+    part(qs.y, qd.y);
+    if (!sure) return false;
+    s = qs;
+    d = qd;
     return true;
 }
 
@@ -323,16 +393,14 @@ __host__ __device__ __forceinline__ IX ins00(IX j, unsigned lo, unsigned hi)
 #endif
 constexpr int ITEMS = QSLC_ITEMS;
 // The easy form (PAT_LEAN) has its own shape: items per iteration for pair
-// gates, Hadamard and diagonal gates, and CTAs of 256 threads per SM.
+// gates and diagonal gates, and CTAs of 256 threads per SM.
 // Measured on a dense 28-qubit state, TB/s of algorithmic bytes, rotateX /
 // phase: 1 item 6.12 / 5.23, 2 items 6.62 / 5.56, 3 items 6.53 / 5.79, 4
 // items - / 6.11 (four CTAs); rotateX with 2 items 6.25 on three CTAs and
-// 6.43 on five.  Hadamard ran 6.34 with one item and 4.09 with two.
+// 6.43 on five.  Hadamard of a 26-qubit state takes 332 us with two items, 370
+// with one.
 #ifndef QSLC_LEAN_ITEMS
 #define QSLC_LEAN_ITEMS 2
-#endif
-#ifndef QSLC_LEAN_ITEMS_H
-#define QSLC_LEAN_ITEMS_H 1
 #endif
 #ifndef QSLC_LEAN_ITEMS_D
 #define QSLC_LEAN_ITEMS_D 4
@@ -368,16 +436,16 @@ constexpr unsigned PAT_ROT = 0x959595u;
 constexpr unsigned PAT_H = 0u;
 constexpr unsigned PAT_DIAG = 0x090909u;
 
-// The general update of the operands that the easy forms leave.  Operands that are all +0 (most of a sparse
-// state) only need the signs of their zeros, which follow from the signs of
-// the coefficients: a sum of two zeros is -0 when both are, a difference p - q
-// when p is -0 and q is +0.  That holds for finite coefficients: those of an
+// The operands that the easy form leaves: first the form with zeros, then the
+// general update.  Operands that are all +0 (most of a sparse state) only
+// need the signs of their zeros, which follow from the signs of the
+// coefficients, easy or not.  That holds for finite coefficients: those of an
 // infinite or NaN angle are NaN, and so is their product with a zero.
 //
-// The sweeps of several gates call it out of line (pair_slow and the like):
-// inline, once per gate type and pair, it would double their code.  There the
-// coefficients go by address (of a kernel parameter): by value they would take
-// registers and stack of every thread.  The sweeps of one gate have it
+// The sweeps of several gates call the general update out of line (pair_slow and
+// the like): inline, once per gate type and pair, it would double their code.
+// There the coefficients go by address (of a kernel parameter): by value they
+// would take registers and stack of every thread.  The sweeps of one gate have it
 // inline, where it costs them less than the call's registers: measured at 26
 // qubits, controlRotateX 201 against 212 us.
 struct SlowCoef {          // the first members of a Coef<double>
@@ -398,18 +466,14 @@ __device__ __forceinline__ Coef<double> general_coef(const SlowCoef *q)
     k.ms = q->ms;
     return k;
 }
-__device__ __forceinline__ double zero_of(uint32_t sign)
-{
-    return __hiloint2double(int(sign & 0x80000000u), 0);
-}
 __device__ __forceinline__ bool plus_zero(const double2 &a)
 {
     return (emu::dbits(a.x) | emu::dbits(a.y)) == 0;
 }
 // Whether c and s are finite; the sine and cosine of one angle are finite together.
-__device__ __forceinline__ bool finite_coef(const Coef<double> &k)
+__device__ __forceinline__ bool finite_coef(const SlowCoef *q)
 {
-    return (__double2hiint(k.c) & 0x7FF00000) != 0x7FF00000;
+    return (__double2hiint(q->c) & 0x7FF00000) != 0x7FF00000;
 }
 
 struct Pair {
@@ -418,43 +482,37 @@ struct Pair {
 template <int OP>
 __device__ __forceinline__ Pair pair_general(double2 a0, double2 a1, const SlowCoef *q)
 {
-    const Coef<double> k = general_coef(q);
-    if (plus_zero(a0) & plus_zero(a1) & finite_coef(k)) {
-        const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
-        const double add = zero_of(c & s), sub = zero_of(c & ~s);
-        if constexpr (OP == P_RX) a0 = a1 = make_double2(add, sub);
-        else if constexpr (OP == P_RY) {
-            a0 = make_double2(sub, sub);
-            a1 = make_double2(add, add);
-        } else {
-            a0 = make_double2(add, sub);
-            a1 = make_double2(sub, add);
-        }
+    if (plus_zero(a0) & plus_zero(a1) & finite_coef(q)) {
+        const uint32_t c = uint32_t(__double2hiint(q->c)), s = uint32_t(__double2hiint(q->s));
+        pair_turns<OP>(a0, a1, [&](double &u, double &v) { turn_signs<true>(u, v, c, s); },
+                       [&](double &u, double &v) { turn_signs<false>(u, v, c, s); });
     } else {
-        pair_update<double, OP>(a0, a1, k, PAT_ROT & 0xFFu);
+        pair_update<double, OP>(a0, a1, general_coef(q), PAT_ROT & 0xFFu);
     }
     return Pair{a0, a1};
 }
-__device__ __forceinline__ Pair hadamard_general(double2 a0, double2 a1, double r, const emu::DivConst *kd)
+__device__ __forceinline__ Pair quotients_general(double2 s, double2 d, double r, const emu::DivConst *kd)
 {
-    Coef<double> k{};
-    k.c = r;
-    k.kd = *kd;
-    // +0 +- +0 is +0, and so is its quotient
-    if (!(plus_zero(a0) & plus_zero(a1))) pair_update<double, P_H>(a0, a1, k, PAT_H & 0xFFu);
-    return Pair{a0, a1};
+    auto quotient = [&](double x) {
+        bool ok = kd->usable != 0;
+        if (ok) {
+            const uint64_t q = emu::div_fast(emu::dbits(x), *kd, ok);
+            if (ok) return emu::dfrom(q);
+        }
+        return __ddiv_rn(x, r);
+    };
+    return Pair{make_double2(quotient(s.x), quotient(s.y)), make_double2(quotient(d.x), quotient(d.y))};
 }
 // x c - y s, y c + x s (INV: s with its sign flipped)
 template <bool INV>
 __device__ __forceinline__ double2 phase_general(double2 a, const SlowCoef *q)
 {
-    const Coef<double> k = general_coef(q);
     const double x = a.x, y = a.y;
-    if (plus_zero(a) & finite_coef(k)) {
-        const uint32_t c = uint32_t(__double2hiint(k.c)), s = uint32_t(__double2hiint(k.s));
-        const double add = zero_of(c & s), sub = zero_of(c & ~s);
-        return INV ? make_double2(add, sub) : make_double2(sub, add);
+    if (plus_zero(a) & finite_coef(q)) {
+        turn_signs<INV>(a.x, a.y, uint32_t(__double2hiint(q->c)), uint32_t(__double2hiint(q->s)));
+        return a;
     }
+    const Coef<double> k = general_coef(q);
     a.x = dot2m<double, !INV>(PAT_DIAG & 3u, x, k.c, k.kc, k.mc, y, k.s, k.ks, k.ms);
     a.y = dot2m<double, INV>((PAT_DIAG >> 2) & 3u, y, k.c, k.kc, k.mc, x, k.s, k.ks, k.ms);
     return a;
@@ -465,9 +523,9 @@ __device__ __noinline__ Pair pair_slow(double2 a0, double2 a1, const SlowCoef *q
 {
     return pair_general<OP>(a0, a1, q);
 }
-static __device__ __noinline__ Pair hadamard_slow(double2 a0, double2 a1, double r, const emu::DivConst *kd)
+static __device__ __noinline__ Pair quotients_slow(double2 s, double2 d, double r, const emu::DivConst *kd)
 {
-    return hadamard_general(a0, a1, r, kd);
+    return quotients_general(s, d, r, kd);
 }
 template <bool INV>
 __device__ __noinline__ double2 phase_slow(double2 a, const SlowCoef *q)
@@ -476,18 +534,47 @@ __device__ __noinline__ double2 phase_slow(double2 a, const SlowCoef *q)
 }
 
 // A gate's update of a pair or of one amplitude: the easy form where it runs,
-// else the general one, out of line, with the coefficients at `q` (`kd` for
-// Hadamard).
-template <int OP>
+// else the form with zeros, else the general one, out of line for CALL, with the
+// coefficients at `q` (`kd` for Hadamard).  Two gates of a 26-qubit state whose
+// imaginary parts are zero, us, on the general split without easy operands / with
+// the easy form and the general call only / with zeros: rotateY 764, 934, 457;
+// Hadamard 539, 1068, 550.  rotateZ leaves out the form with zeros where the
+// general one is a call: it meets zeros in single lanes beside easy ones, which
+// then run both (1093 us with it, 725 without).
+template <int OP, bool CALL = true>
 __device__ __forceinline__ void pair_either(double2 &a0, double2 &a1, const Coef<double> &k, const SlowCoef *q,
                                             const emu::DivConst *kd)
 {
-    if (pair_lean<OP>(a0, a1, k)) return;
-    Pair r;
-    if constexpr (OP == P_H) r = hadamard_slow(a0, a1, k.c, kd);
-    else r = pair_slow<OP>(a0, a1, q);
-    a0 = r.a0;
-    a1 = r.a1;
+    if constexpr (OP == P_H) {
+        double2 s = make_double2(__dadd_rn(a0.x, a1.x), __dadd_rn(a0.y, a1.y));
+        double2 d = make_double2(__dsub_rn(a0.x, a1.x), __dsub_rn(a0.y, a1.y));
+        // opaque from here: the compiler would otherwise compute the sums a
+        // second time after the test, and the FP64 pipe is what binds
+        asm volatile("" : "+d"(s.x), "+d"(s.y), "+d"(d.x), "+d"(d.y));
+        if (!quotients_lean(s, d, k.ld) && !quotients_zeros(s, d, k.ld)) {
+            const Pair r = CALL ? quotients_slow(s, d, k.c, kd) : quotients_general(s, d, k.c, kd);
+            s = r.a0;
+            d = r.a1;
+        }
+        a0 = s;
+        a1 = d;
+    } else if (!pair_lean<OP>(a0, a1, k.lc, k.ls) && !((!CALL || OP != P_RZ) && pair_zeros<OP>(a0, a1, k.lc, k.ls))) {
+        const Pair r = CALL ? pair_slow<OP>(a0, a1, q) : pair_general<OP>(a0, a1, q);
+        a0 = r.a0;
+        a1 = r.a1;
+    }
+}
+template <bool INV, bool CALL = true>
+__device__ __forceinline__ void phase_either(double2 &a, const Coef<double> &k, const SlowCoef *q)
+{
+    if (!phase_lean<INV>(a, k.lc, k.ls) && !phase_zeros<INV>(a, k.lc, k.ls))
+        a = CALL ? phase_slow<INV>(a, q) : phase_general<INV>(a, q);
+}
+// phase_either with the sign of s chosen at run time.
+__device__ __forceinline__ void phase_flip(double2 &a, uint32_t flip, const Coef<double> &k, const SlowCoef *q)
+{
+    if (!phase_lean<false>(a, k.lc, k.ls, flip) && !phase_zeros<false>(a, k.lc, k.ls, flip))
+        a = flip ? phase_slow<true>(a, q) : phase_slow<false>(a, q);
 }
 
 // The same for the sweeps of one gate, whose coefficients are a kernel
@@ -496,25 +583,16 @@ __device__ __forceinline__ void pair_either(double2 &a0, double2 &a1, const Coef
 template <class T, int OP, bool LEAN>
 __device__ __forceinline__ void pair_gate(cplx<T> &a0, cplx<T> &a1, const Coef<T> &k, unsigned md)
 {
-    if constexpr (LEAN && sizeof(T) == 8 && OP != P_SWAP && OP != P_Y) {
-        if (pair_lean<OP>(a0, a1, k)) return;
-        Pair r;
-        if constexpr (OP == P_H) r = hadamard_general(a0, a1, k.c, &k.kd);
-        else r = pair_general<OP>(a0, a1, slow_coef(k));
-        a0 = r.a0;
-        a1 = r.a1;
-    } else {
+    if constexpr (LEAN && sizeof(T) == 8 && OP != P_SWAP && OP != P_Y)
+        pair_either<OP, false>(a0, a1, k, slow_coef(k), &k.kd);
+    else
         pair_update<T, OP>(a0, a1, k, md);
-    }
 }
 template <class T, int OP, bool LEAN>
 __device__ __forceinline__ void diag_gate(cplx<T> &a, const Coef<T> &k, unsigned md)
 {
-    if constexpr (LEAN && sizeof(T) == 8 && OP != D_NEG) {
-        if (!phase_lean<OP>(a, k)) a = phase_general<OP == D_PHASE_INV>(a, slow_coef(k));
-    } else {
-        diag_update<T, OP>(a, k, md);
-    }
+    if constexpr (LEAN && sizeof(T) == 8 && OP != D_NEG) phase_either<OP == D_PHASE_INV, false>(a, k, slow_coef(k));
+    else diag_update<T, OP>(a, k, md);
 }
 
 // The mask of item r (the pattern repeats after three) of a sweep compiled
@@ -530,7 +608,6 @@ constexpr unsigned pair_pattern() { return OP == P_H ? PAT_H : PAT_ROT; }
 
 template <unsigned CPAT, int LEAN_ITEMS>
 constexpr int sweep_items() { return CPAT == PAT_LEAN ? LEAN_ITEMS : ITEMS; }
-constexpr int pair_items(int op) { return op == P_H ? QSLC_LEAN_ITEMS_H : QSLC_LEAN_ITEMS; }
 
 // Launch `f(std::integral_constant<unsigned, P>{})` with P = PAT_LEAN when
 // `lean`, else 0 when pat is 0 (all on the FP64 pipe), else PAT_RUNTIME.
@@ -558,8 +635,8 @@ Coef<T> coef(T c, T s)
     k.mc = emu::make_mulk(double(c));
     k.ms = emu::make_mulk(double(s));
     k.kd = emu::make_div(double(c));
-    k.lc = emu::make_lean(double(c));
-    k.ls = emu::make_lean(double(s));
+    k.lc = emu::make_lean_gate(double(c));
+    k.ls = emu::make_lean_gate(double(s));
     k.ld = emu::make_lean_div(double(c));
     return k;
 }

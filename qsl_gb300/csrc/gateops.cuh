@@ -21,7 +21,7 @@ template <class T>
 __device__ __forceinline__ void group_phase(cplx<T> &a, const Coef<T> &k)
 {
     if constexpr (sizeof(T) == 8) {
-        if (!phase_lean<D_PHASE>(a, k)) a = phase_slow<false>(a, slow_coef(k));
+        phase_either<false>(a, k, slow_coef(k));
     } else {
         diag_update<T, D_PHASE>(a, k);
     }

@@ -37,7 +37,7 @@ template <class T, int OP, unsigned CPAT = PAT_RUNTIME, class IX = uint64_t>
 __global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair1(cplx<T> *__restrict__ st, uint64_t npairs,
                                                unsigned t, const __grid_constant__ Coef<T> k, unsigned pat)
 {
-    constexpr int N = sweep_items<CPAT, pair_items(OP)>();
+    constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS>();
     const IX bit = IX(1) << t;
     const IX stride = IX(gridDim.x) * blockDim.x;
     for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(npairs); j += N * stride) {
@@ -238,7 +238,7 @@ __global__ void QSLC_LEAN_BOUNDS(CPAT) k_pair2(cplx<T> *__restrict__ st, uint64_
                                                unsigned lo, unsigned hi, uint64_t b1,
                                                uint64_t b2, const __grid_constant__ Coef<T> k, unsigned pat)
 {
-    constexpr int N = sweep_items<CPAT, pair_items(OP)>();
+    constexpr int N = sweep_items<CPAT, QSLC_LEAN_ITEMS>();
     const IX stride = IX(gridDim.x) * blockDim.x;
     for (IX j = IX(blockIdx.x) * blockDim.x + threadIdx.x; j < IX(nquads); j += N * stride) {
         cplx<T> a0[N], a1[N];

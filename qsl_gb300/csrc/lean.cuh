@@ -8,7 +8,8 @@
 // the caller, which tests them first (easy_range, easy_product) and sends a
 // thread through the general path when it has one that is not easy.  What the
 // restriction buys:
-//   - no zero handling, and no rounding ties: a product lies half-way
+//   - no zero handling (LeanOpZ adds it, for the threads that need it), and
+//     no rounding ties: a product lies half-way
 //     between two doubles only when the operand's significand has at least
 //     32 trailing zeros (see make_lean), so the sticky bits are not needed;
 //   - the shift moves before the product: whether ma * mc reaches 2^105 is
@@ -68,6 +69,16 @@ QSLC_HD LeanK make_lean(double c)
     return r;
 }
 
+// The same for a gate's constants, powers of two included (the sines and cosines
+// of quarter turns): a product by a power of two keeps the operand's significand,
+// so it is never a tie.
+QSLC_HD LeanK make_lean_gate(double c)
+{
+    LeanK r = make_lean(c);
+    r.usable |= make_mulk(c).usable && (dbits(c) & MANT) == 0;
+    return r;
+}
+
 // The parts of an easy operand that its products share.
 struct LeanOp {
     uint32_t lo, hi;      // ma << 2
@@ -110,6 +121,35 @@ QSLC_HD bool easy_range(uint64_t a)
     return (ahi + ahi) - 2 * PACK_EF_LO20 <= 2 * PACK_EF_SPAN20 + 0x001FFFFFu;
 }
 QSLC_HD bool easy_product(uint64_t a) { return easy_range(a) & (uint32_t(a) != 0); }
+
+// ---- zeros --------------------------------------------------------------------
+// An operand that is easy or a zero of either sign.  A zero has a significand
+// of 0 and an exponent of 0: its product has no significand either, and the sign
+// alone where the constant's exponent is left out.
+struct LeanOpZ {
+    LeanOp op;
+    bool zero;
+};
+
+// By words: the compiler turns a test of the whole into a comparison on the FP64
+// pipe, which the sums need (8 comparisons beside the 4 sums of a pair).
+QSLC_HD bool is_zero(uint64_t a)
+{
+    const uint32_t ahi = uint32_t(a >> 32);
+    return ((ahi + ahi) | uint32_t(a)) == 0;
+}
+
+QSLC_HD LeanOpZ lean_operand_z(uint64_t a)
+{
+    LeanOpZ o;
+    o.op = lean_operand(a);
+    o.zero = is_zero(a);
+    if (o.zero) o.op.hi = 0;
+    return o;
+}
+
+// The sign of a constant, in place: its exponent's part of k is negative.
+QSLC_HD uint32_t lean_sign(const LeanK &c) { return ~c.k & 0x80000000u; }
 
 // ---- squares ------------------------------------------------------------------
 // m * m of a significand m lies in [2^104, 2^106).  It is half-way between two
@@ -158,12 +198,12 @@ QSLC_HD uint64_t round96(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t s0, uin
 #endif
 }
 
-// RN(a * c), packed.
-QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c)
+// RN(a * c), packed; k0: the constant's sign and exponent.
+QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c, uint32_t k0)
 {
     const bool top = ((uint64_t(a.hi) << 32) | a.lo) >= ((uint64_t(c.t1) << 32) | c.t0);
     const uint32_t c0 = top ? c.h0 : c.l0, c1 = top ? c.h1 : c.l1;
-    const uint32_t k = c.k + a.se + (top ? 0x00100000u : 0u);
+    const uint32_t k = k0 + a.se + (top ? 0x00100000u : 0u);
     // partial sums stay below 2^64: c1 < 2^31, a.hi < 2^23
     const uint64_t mid = mulwide(a.hi, c0) + (mulwide(a.lo, c1) + 0x80000000u);
     const uint64_t high = mulwide(a.hi, c1);
@@ -171,6 +211,8 @@ QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c)
     return round96(uint32_t(mid), uint32_t(high), uint32_t(high >> 32), mulhi32(a.lo, c0), uint32_t(mid >> 32), k,
                    rest);
 }
+QSLC_HD uint64_t lean_mul(const LeanOp &a, const LeanK &c) { return lean_mul(a, c, c.k); }
+QSLC_HD uint64_t lean_mul(const LeanOpZ &a, const LeanK &c) { return lean_mul(a.op, c, a.zero ? lean_sign(c) : c.k); }
 
 // A divisor fixed for a whole kernel: the reciprocals 2^146 / my (for
 // mx >= my) and 2^147 / my (for mx < my), rounded down, as three words.

@@ -124,7 +124,7 @@ __device__ __forceinline__ void run_pairs(double2 (&v)[A], unsigned set, const C
 
 __device__ __forceinline__ void run_rotate(double2 &a, uint32_t flip, const Coef<double> &k, const SlowCoef *q)
 {
-    if (!phase_flip_lean(a, flip, k)) a = flip ? phase_slow<true>(a, q) : phase_slow<false>(a, q);
+    phase_flip(a, flip, k, q);
 }
 
 template <int A, int NG>
