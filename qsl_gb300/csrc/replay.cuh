@@ -18,7 +18,7 @@
 //   the running sum crosses a power of two) are replayed term by term.
 //
 // Everything here is __host__ __device__ so the same code runs in the
-// kernels and in the host sequencer.
+// kernels and in its host tests.
 #pragma once
 
 #include <cstdint>
@@ -271,28 +271,6 @@ QSLC_HD float norm2_rn(float re, float im)
     volatile float b = im * im;
     return a + b;
 #endif
-}
-
-// Error-free double-double accumulation (Knuth's TwoSum); only an estimate
-// of the exact prefix is needed, to guess each tile's binade.
-struct dd {
-    double hi, lo;
-};
-QSLC_HD dd dd_add(dd a, double b)
-{
-    double s = a.hi + b;
-    double bb = s - a.hi;
-    double err = (a.hi - (s - bb)) + (b - bb);
-    double lo = a.lo + err;
-    double hi = s + lo;
-    return dd{hi, lo - (hi - s)};
-}
-QSLC_HD dd dd_add(dd a, dd b)
-{
-    dd r = dd_add(a, b.hi);
-    r.lo += b.lo;
-    double hi = r.hi + r.lo;
-    return dd{hi, r.lo - (hi - r.hi)};
 }
 
 }  // namespace qslc
