@@ -17,10 +17,10 @@
 // diagonal gates are tested on the indices.
 //
 // complex64 sweeps are bound by HBM one gate at a time, and runs by
-// instructions: 17 gates of a 25-qubit circuit take 300 us a run, 80 of them
-// the traffic (four such layers: 5.6 ms before, 2.7 ms).  complex128 runs
-// are bound by the FP64 and ALU pipes as the single sweeps are, and gain where
-// launches or moves count: 8 layers of 10 qubits 418 -> 203 us.
+// instructions: four layers of a 25-qubit circuit take 2.3 ms, 5.6 ms with a
+// sweep for two gates.  complex128 runs are bound by the FP64 and ALU pipes as the
+// single sweeps are, and gain where launches or moves count: 8 layers of 10
+// qubits, 120 calls, 418 -> 165 us.
 #include "bounds.cuh"
 #include "gatemath.cuh"
 
@@ -345,27 +345,30 @@ struct Shape {
 // and a gate takes the time that one warp needs for its amplitudes, about 8
 // clocks an instruction: fewer amplitudes a thread, in more warps, are quicker
 // although the targets of a run then take more steps.  Circuits of 8 layers, us,
-// usual and small: complex128 of 6 qubits 166 and 135, of 10 258 and 225, of 14
-// 308 and 255, of 17 384 and 317 (to 19 qubits, where runs_any ends); complex64 of 6 qubits 121 and 107, of 12 235
-// and 216, of 14 228 and 232.
-template <class T> constexpr unsigned SMALL_STATE = sizeof(T) == 8 ? 19 : 13;
+// usual and small: complex128 of 6 qubits 140 and 106, of 10 195 and 162, of 14
+// 275 and 214, of 17 372 and 308, of 18 462 and 428, of 19 626 and 716; complex64
+// of 6 qubits 96 and 87, of 12 172 and 163, of 14 (usual) 197.
+template <class T> constexpr unsigned FEW_REGS = sizeof(T) == 8 ? 18 : 13;
 template <class T> int reg_bits(const qslc_state *s)
 {
-    return s->n <= SMALL_STATE<T> ? SMALL_REG_BITS<T> : REG_BITS<T>;
+    return s->n <= FEW_REGS<T> ? SMALL_REG_BITS<T> : REG_BITS<T>;
 }
+
+// complex128 states of this many qubits take runs of everything (runs_any).
+constexpr unsigned SMALL_STATE = 19;
 
 // Small states take small tiles: many CTAs share the arithmetic, which a run
 // of few gates does not fill otherwise.  Circuits of 8 layers on one GB300,
-// us, tiles of 2^7 / 2^8 / 2^9 / 2^10 amplitudes: complex128 of 10 qubits 229 /
-// 217 / 225 / 297, of 14 261 / 248 / 255 / 355, of 17 329 / 316 / 317 / 437;
-// complex64 of 10 qubits 217 / 192 / 196 / 186, of 14 256 / 230 / 232 / 219,
-// of 25 (4 layers) 3044 with 2^10, 2871 with 2^11 and 2655 with 2^12.  Two
-// contiguous low qubits were never slower than three or four: the others are
-// left to the run.
+// us, tiles of 2^7 / 2^8 / 2^9 / 2^10 amplitudes: complex128 of 10 qubits 167 /
+// 162 / 162 / 235, of 14 231 / 218 / 215 / 308, of 17 325 / 308 / 297 / 387, of 19
+// with 2^8 627, with 2^11 748; complex64 of 10 qubits 145 / 140 / 135 / 129, of 14
+// 215 / 201 / 200 / 192, of 25 (4 layers) 3044 with 2^10, 2871 with 2^11 and 2655
+// with 2^12.  Two contiguous low qubits were never slower than three or four: the
+// others are left to the run.
 Shape shape_of(const qslc_state *s)
 {
     const bool dbl = s->dtype == QSLC_C128;
-    const unsigned b = std::min(dbl ? (s->n > SMALL_STATE<double> ? 11u : 8u) : (s->n >= 20 ? 12u : 10u), s->n);
+    const unsigned b = std::min(dbl ? (s->n > SMALL_STATE ? 11u : 8u) : (s->n >= 20 ? 12u : 10u), s->n);
     const unsigned r = unsigned(dbl ? reg_bits<double>(s) : reg_bits<float>(s));
     const unsigned t = b >= r + 8 ? 256 : b > r + 5 ? 1u << (b - r) : 32;
     return Shape{b, std::min(b, 2u), std::min(t, 1u << b)};
@@ -635,10 +638,10 @@ bool is_move(int code)
 // arithmetic binds, and a rotation takes 1.71 clocks per amplitude and SM in a
 // run (coefficients read per gate, a barrier per two gates) against 1.29 in
 // k_group2.  Circuits of 8 layers, us, pairs with runs of moves beside them
-// against runs of everything: of rotations and all two-qubit gates, 18 qubits
-// 702 and 462, 19 qubits 949 and 785; of rotations and controlNots, 18 qubits
-// 591 and 460, 19 qubits 852 and 822, 20 qubits 1231 and 1514.
-bool runs_any(const qslc_state *s) { return s->dtype == QSLC_C64 || s->n <= SMALL_STATE<double>; }
+// against runs of everything: of one-qubit gates and all two-qubit gates, 18 qubits
+// 796 and 504, 19 qubits 1090 and 835; of one-qubit gates and controlNots, 18 qubits
+// 682 and 428, 19 qubits 919 and 627, 20 qubits 1209 and 1248.
+bool runs_any(const qslc_state *s) { return s->dtype == QSLC_C64 || s->n <= SMALL_STATE; }
 
 // Whether one run is quicker than the gates' own sweeps, by the share of the
 // state that each moves (in quarters of a read and write of all of it) and,
