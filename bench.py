@@ -84,8 +84,8 @@ def kernel_of(gate: str) -> str:
 # so next to the number, and --traffic replaces it with a capture's figure.
 K_PAIR1_TRAFFIC_RATIO = 2.086 / 2.147
 # The same for the grouped sweep of two rotations on a dense 26-qubit state:
-# 1.074 + 1.033 GB of DRAM traffic for the two gates' 2 x 2.147 GB.
-K_GROUP2_TRAFFIC_RATIO = (1.074 + 1.033) / (2 * 2.147)
+# 1.074 + 1.024 GB of DRAM traffic for the two gates' 2 x 2.147 GB.
+K_GROUP2_TRAFFIC_RATIO = (1.074 + 1.024) / (2 * 2.147)
 
 
 def peaks():
@@ -574,7 +574,7 @@ def roofline_of(args, name, top, peak, peak_kind):
     elif name == "k_group2":
         out["traffic"] = per_launch * K_GROUP2_TRAFFIC_RATIO
         out["traffic_source"] = ("scaled from an earlier ncu capture of k_group2 (two rotations) on a dense "
-                                 "26-qubit state (DRAM bytes / algorithmic bytes of both gates = 0.491: one "
+                                 "26-qubit state (DRAM bytes / algorithmic bytes of both gates = 0.489: one "
                                  "read and one write of the state); not measured in this run")
     else:
         out["traffic"] = None

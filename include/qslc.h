@@ -151,7 +151,10 @@ QSLC_API int qslc_set_basis(qslc_state *s, uint64_t index);
 QSLC_API int qslc_gate1(qslc_state *s, int gate, unsigned targ, double angle);
 
 /* Two-qubit gate (gates.cpp:215-682; np/gates.cpp:118-415).  EINVAL when
- * q1 == q2 or either index is out of range. */
+ * q1 == q2 or either index is out of range.  On a plain state it may be held
+ * back as one-qubit gates are: call qslc_flush before ordering other work
+ * after the handle's stream, by an event say.  A failure of a held gate's launch
+ * is reported by the call that applies it. */
 QSLC_API int qslc_gate2(qslc_state *s, int gate, unsigned q1, unsigned q2, double angle);
 
 /* prob(targ, outcome) (measure.cpp:126-147; np/measure.cpp:141-168).  The

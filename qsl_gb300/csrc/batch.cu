@@ -16,7 +16,7 @@
 // The graph holds four kernels.  k_batch runs the circuits and leaves every
 // instance's |a|^2 terms in global memory; k_batch_probs64 (or 32) and k_batch_cdf, side
 // by side, turn them into the probabilities (chains of dependent adds, one
-// per thread) and the shots; k_batch_sort, beside k_batch, sorts each
+// per thread) and the shots; k_batch_sort, before k_batch, sorts each
 // instance's uniforms for the CDF walk.
 //
 // Schedule of k_batch: persistent clusters of CTAs pull instances, largest
@@ -892,7 +892,7 @@ struct qslc_batch {
 
 namespace {
 
-// The arena holds two buffers of 2^nmax amplitudes per CTA; beyond this
+// The arena holds two buffers of 2^nmax amplitudes per cluster; beyond this
 // many bytes the grid shrinks instead.
 constexpr uint64_t ARENA_CAP = uint64_t(64) << 30;
 

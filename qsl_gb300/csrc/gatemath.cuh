@@ -207,7 +207,7 @@ __device__ __forceinline__ void diag_update(cplx<T> &a, const Coef<T> &k, unsign
 // no mask is known that names exactly the lanes of a vote.
 //
 // Bound by the FP64 pipe (two operations per SM and clock) and the ALU pipe
-// together: 96 instructions per amplitude and gate against 150 with the
+// together: 100 instructions per amplitude and gate against 150 with the
 // general split "PPPQ", 2 of them FP64 instead of 2.7.  Two rotateX gates of a
 // 26-qubit dense state in one sweep: 761 us with the general split, 550 us
 // with this; FP64 pipe 79% busy.

@@ -78,8 +78,9 @@ struct ProdAll {         // every amplitude, ascending
 // whose parts are all easy (lean.cuh) takes squares on the integer pipes, about
 // 20 instructions each.  k_seq_steps leaves the pipe the other square and the
 // sum (BOTH false): with the sum alone its ALU pipe, which counts the grid steps,
-// is 80% busy and the FP64 pipe 31%.  Over all 2^28 amplitudes 740 us with no
-// square on the integer pipes, 660 with both, 608 with one.  The walk, one CTA
+// is the fuller one.  Over all 2^28 amplitudes of a dense state 1649 us with no
+// square on the integer pipes, 1306 with both, 1205 with one; over half of them
+// 653 with one, 735 for the three lowest qubits.  The walk, one CTA
 // that waits for its terms, leaves the sum alone: 138 -> 126 us at 20 qubits.
 template <bool BOTH, int N>
 __device__ __forceinline__ void norms(const float2 (&a)[N], float (&p)[N])
@@ -250,11 +251,11 @@ __global__ void __launch_bounds__(SEQ_GUESS_TPB) k_seq_guess(const double *__res
 // a rounding tie; a warp with a tie does its piece again, composing the terms
 // in order.
 //
-// Bound by the FP64 pipe (three operations a term, 74% busy) with
-// the integer work on step counts behind it.  Two passes over the state with the sums
-// of the first in FP64, a host step between them and 32-way conflicts in shared
-// memory took 2.3 ms for the probability of one qubit of 28; this and the
-// redone tiles take 1.0.
+// Bound by the FP64 pipe (a square and the sum a term, 69% busy) and the ALU
+// pipe (the other square, the step counts, 68%) together, at 0.46 of HBM.  Two
+// passes over the state with the sums of the first in FP64, a host step between
+// them and 32-way conflicts in shared memory took 2.3 ms for the probability of
+// one qubit of 28; this and the redone tiles take 0.7.
 // ---------------------------------------------------------------------------
 // Packs a term's grid steps with its tie bit (bit 63); steps never reach
 // 2^62 without also raising `big`.
