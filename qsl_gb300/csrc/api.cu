@@ -175,10 +175,14 @@ int check_handle(const qslc_state *s)
 }
 
 // What is queued on `later` from here on runs after what is queued on
-// `earlier` so far.
+// `earlier` so far.  Work captured from `earlier` runs when its graph does, which
+// is the caller's to order: an event of it would draw `later` into the capture.
 int order_after(cudaStream_t later, cudaStream_t earlier)
 {
     if (later == earlier) return QSLC_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    QSLC_CUDA(cudaStreamIsCapturing(earlier, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return QSLC_OK;
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e == cudaSuccess) {

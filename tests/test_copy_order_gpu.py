@@ -35,3 +35,26 @@ def test_the_source_may_change_at_once(qsl, kind, change):
         del view, src
     dst.synchronize()
     assert torch.equal(dst.device_view(), want)
+
+
+def test_assign_may_be_captured(qsl):
+    """Captured from the destination's stream, the copy is one of the source as
+    it is at each replay; the source's stream stays out of the capture."""
+    import torch
+    n = 12
+    src, dst = qsl.Qubits(n), qsl.Qubits(n)
+    stream = torch.cuda.Stream()
+    dst.set_stream(stream.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        dst.assign(src)
+        src.gate("hadamard", 0, None, 0.0)      # runs at once
+        src.flush()
+    for t in range(n):
+        src.gate("rotateX", t, None, 0.3 + t)
+        src.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = src.getState()
+        assert t or np.count_nonzero(want) == 2     # the Hadamard, and rotateX on its qubit
+        assert np.array_equal(dst.getState().view(np.uint64), want.view(np.uint64))
